@@ -49,10 +49,10 @@ Moe::Moe(const ne_moe_desc &d, int max_rows_) : desc(d), max_rows(max_rows_) {
   raw_sgu = (float *)al(Sg * R * 2 * I * 4);
   raw_d = (float *)al(Sd * P * H * 4);
   raw_sd = (float *)al(Sd * R * H * 4);
-  xh_gu = (__half *)al(P * 2 * H * 2 * A_HALFS_PER_INPUT);
-  xh_sgu = (__half *)al(R * 2 * H * 2 * A_HALFS_PER_INPUT);
-  xh_d = (__half *)al(P * I * 2 * A_HALFS_PER_INPUT);
-  xh_sd = (__half *)al(R * I * 2 * A_HALFS_PER_INPUT);
+  xh_gu = (__half *)al(P * 2 * H * 2);
+  xh_sgu = (__half *)al(R * 2 * H * 2);
+  xh_d = (__half *)al(P * I * 2);
+  xh_sd = (__half *)al(R * I * 2);
   gush = (float *)al(R * 2 * I * 4);
   if (shared_q8) { q8_g = (float *)al(R * I * 4); q8_u = (float *)al(R * I * 4); q8_act = (float *)al(R * I * 4); }
   sho = (float *)al(R * H * 4);
@@ -146,7 +146,7 @@ MoeParams Moe::params(const float *x, int rows, float *y) {
   p.H = desc.hidden; p.I = desc.inter; p.E = desc.experts; p.topk = desc.top_k;
   p.Kx = desc.k_expert; p.Ks = desc.k_shared;
   p.e0 = desc.expert_first; p.ecount = desc.expert_count;
-  p.rows = rows; p.P = rows * desc.top_k; p.has_shared = has_shared ? 1 : 0; p.shared_pre = shared_q8 ? 1 : 0; p.dup = g_summand_product;
+  p.rows = rows; p.P = rows * desc.top_k; p.has_shared = has_shared ? 1 : 0; p.shared_pre = shared_q8 ? 1 : 0;
   p.router = (const uint16_t *)desc.router_dev;
   p.sgate = (const uint16_t *)desc.shared_gate_w_dev;
   auto stack = [](const ne_exl3_stack &s) { return Exl3Stack{(const char *)s.trellis_dev, (const __half *)s.suh_dev, (const __half *)s.svh_dev}; };

@@ -124,9 +124,8 @@ __device__ __forceinline__ void dec8(uint32_t w0, uint32_t w1, uint32_t w2, uint
   }
 }
 
-// The same 8 slots left as their summand pairs: r[t] = (lo, hi) with weight = fp16(lo + hi). The stream kernels build the
-// tensor-core operand from these words directly (one half add per word for the exact weight, none for the opt-in summand
-// product), so the pack of dec8 (two weights per register) is not executed.
+// The same 8 slots left as their summand pairs: r[t] = (lo, hi) with weight = fp16(lo + hi). The stream kernels round and
+// pack these on the tensor core (round_pairs), so the half adds and the pack of dec8 are not executed.
 template <int K>
 __device__ __forceinline__ void dec8_raw(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t a, const McgConst &c, uint32_t (&r)[8]) {
   if constexpr (Codec<K>::UNIFORM) {
@@ -155,16 +154,24 @@ __device__ __forceinline__ void dec8_raw(uint32_t w0, uint32_t w1, uint32_t w2, 
   }
 }
 
-// Layout of a prepared activation row (the B operand of the stream kernels) for that product: per k-tile of 16 inputs
-// 32 halfs = 16 pairs in the order inputs 0, 2, .. 14, then 1, 3, .. 15, so that one ldmatrix.x4 of an 8-row group
-// yields the even-input and the odd-input fragments. A row of n inputs is 2 n halfs. The pair is (v, 0) for the exact
-// product (the kernel feeds (w, w), w = fp16(lo + hi): the accumulator receives w * v) and (v, v) for the summand
-// product (the kernel feeds (lo, hi): lo * v + hi * v).
-constexpr int A_HALFS_PER_INPUT = 2;
-__device__ __forceinline__ void store_a(__half *row, int i, float v, int dup) {
-  const int w = (i >> 4) * 16 + (i & 1) * 8 + ((i & 15) >> 1);
-  const __half h = __float2half_rn(v);
-  reinterpret_cast<__half2 *>(row)[w] = __halves2half2(h, dup ? h : __ushort_as_half((unsigned short)0));
+// Rounding and packing of summand pairs on the tensor core. One mma.m16n8k16 with f16 accumulators multiplies a fragment of
+// pairs (lo, hi) with the constant 0 / 1 matrix that adds the two halves of every pair: its f16 result is fp16(lo + hi) (the
+// two summands are at most three binades apart, so the sum is exact before that one rounding to nearest even: equal to the
+// half add for all 2^15 codewords), and the columns are arranged so that a lane gets back its own two slots packed in one
+// register. In: slots x, y of column c and of column c + 8. Out: d[0] = (x, y) of column c, d[1] of column c + 8, the words of
+// an A fragment. Two of these replace eight half adds (or four pair adds and packs) per tile: 2 instructions for 8 to 12 on
+// the pipes that bound the decode.
+struct PairSum {  // the lane's fragment of the constant matrix: output column 2j adds pair j, 2j + 1 adds pair j + 4
+  uint32_t b0, b1;
+  static __device__ __forceinline__ PairSum make(int lane) {
+    const int g = lane >> 2, q = lane & 3;
+    return PairSum{g == 2 * q ? 0x3C003C00u : 0u, g == 2 * q + 1 ? 0x3C003C00u : 0u};
+  }
+};
+__device__ __forceinline__ void round_pairs(uint32_t (&d)[2], uint32_t xc, uint32_t xc8, uint32_t yc, uint32_t yc8, const PairSum &e) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f16.f16.f16.f16 {%0,%1}, {%2,%3,%4,%5}, {%6,%7}, {%8,%8};"
+      : "=r"(d[0]), "=r"(d[1])
+      : "r"(xc), "r"(xc8), "r"(yc), "r"(yc8), "r"(e.b0), "r"(e.b1), "r"(0u));
 }
 
 // normalised Hadamard of size N (16..128) over a 128-element chunk held by a warp as (lane, lane+32, lane+64, lane+96);

@@ -14,10 +14,10 @@ constexpr int kMinStages = SG_KS >= 16 ? 2 : 3;
 StreamLayout make_layout(int Kmax, int kcmax, int arows, int ctas_per_sm) {
   StreamLayout l;
   l.stage_bytes = SG_KS * SG_WARPS * 32 * Kmax;
-  l.lda = kcmax * 16 * A_HALFS_PER_INPUT + 8;
+  l.lda = kcmax * 16 + 8;
   l.arows = std::max(arows, 1);
   const size_t budget = smem_budget(ctas_per_sm);
-  const size_t base = l.ring_off() + (size_t)l.lda * 2;
+  const size_t base = l.ring_off() + 64;
   const size_t want_stages = SG_KS >= 16 ? 3 : 6;
   // three A slots or more let the producer issue the rows of unit u + 2 while the consumers are still on unit u; the widest
   // row counts only fit two (the producer then waits for the consumers to leave unit u - 1 before it sends unit u + 1)
@@ -37,7 +37,7 @@ int kc_cap(int arows, int Kmax, int ctas) {
   const long room = (long)smem_budget(ctas) - 4096 - (long)kMinStages * SG_KS * SG_WARPS * 32 * Kmax;
   auto cap = [&](int slots) {
     const long halfs_per_row = room / slots / std::max(arows, 1) / 2;
-    return std::max(0, std::min((int)((halfs_per_row - 8) / (16 * A_HALFS_PER_INPUT)) / SG_KS * SG_KS, 256));
+    return std::max(0, std::min((int)((halfs_per_row - 8) / (16)) / SG_KS * SG_KS, 256));
   };
   const int c3 = cap(3);
   return c3 >= SG_KS || ctas > 1 ? c3 : cap(2);
@@ -83,7 +83,7 @@ LinearPlan plan_linear(int in, int out, int K, int rows) {
 }
 
 __global__ void __launch_bounds__(128) prep_rows_kernel(const float *__restrict__ x, const __half *__restrict__ suh,
-                                                        __half *__restrict__ xh, int rows, int n, int hn, float hscale, int dup) {
+                                                        __half *__restrict__ xh, int rows, int n, int hn, float hscale) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int chunk = blockIdx.x * 4 + warp, r = blockIdx.y;
   pdl_wait();
@@ -99,14 +99,14 @@ __global__ void __launch_bounds__(128) prep_rows_kernel(const float *__restrict_
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const int i = chunk * 128 + lane + 32 * j;
-    if (i < n) store_a(xh + (size_t)r * n * A_HALFS_PER_INPUT, i, v[j], dup);
+    if (i < n) (xh + (size_t)r * n)[i] = __float2half_rn(v[j]);
   }
 }
 
 void launch_prep_rows(const float *x, const __half *suh, __half *xh, int rows, int n, cudaStream_t st) {
   const int hn = had_size(n);
   dim3 grid(((n + 127) / 128 + 3) / 4, rows);
-  launch_pdl(prep_rows_kernel, grid, dim3(128), 0, st, x, suh, xh, rows, n, hn, (float)(1.0 / sqrt((double)hn)), g_summand_product);
+  launch_pdl(prep_rows_kernel, grid, dim3(128), 0, st, x, suh, xh, rows, n, hn, (float)(1.0 / sqrt((double)hn)));
 }
 
 // y[r][c] = (H_ho(sum_s raw[s][r]))[c] * svh[c]; one warp per (row, 128-column chunk), splits summed in index order
@@ -148,7 +148,6 @@ struct MlPtrs {
   float *y[ML_MAX];
   int out[ML_MAX], ho[ML_MAX];
   float hs[ML_MAX];  // 1 / sqrt(ho), rounded once on the host like everywhere else
-  int dup;           // store_a's pair form: the product mode in force when the call was enqueued
 };
 
 __global__ void __launch_bounds__(128) prep_rows_multi_kernel(const float *__restrict__ x, const MlPtrs a, int rows, int n, int hn, float hscale) {
@@ -167,7 +166,7 @@ __global__ void __launch_bounds__(128) prep_rows_multi_kernel(const float *__res
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const int i = chunk * 128 + lane + 32 * j;
-    if (i < n) store_a(a.xh[m] + (size_t)r * n * A_HALFS_PER_INPUT, i, v[j], a.dup);
+    if (i < n) (a.xh[m] + (size_t)r * n)[i] = __float2half_rn(v[j]);
   }
 }
 
@@ -227,7 +226,6 @@ MultiLinearPlan plan_linear_multi(int n, int in, const int *out, const int *K, i
 void launch_linear_multi(const MultiLinearPlan &p, const MultiLinearArgs &a, const float *x, void *scratch, int *status, cudaStream_t st) {
   MultiLinearProblem pr{};
   MlPtrs q{};
-  q.dup = g_summand_product;
   char *cur = (char *)scratch;
   int maxout = 0;
   pr.n = p.n; pr.in = p.in; pr.rows = p.rows; pr.IT = p.IT; pr.S = p.S; pr.kc = p.kc;
@@ -236,7 +234,7 @@ void launch_linear_multi(const MultiLinearPlan &p, const MultiLinearArgs &a, con
     float *raw = (float *)cur;
     cur += (p.raw_floats(m) * 4 + 255) & ~(size_t)255;
     __half *xh = (__half *)cur;
-    cur += ((size_t)p.rows * p.in * A_HALFS_PER_INPUT * 2 + 255) & ~(size_t)255;
+    cur += ((size_t)p.rows * p.in * 2 + 255) & ~(size_t)255;
     make_trellis_map(&pr.maps[m], a.trellis[m], 1, p.IT, p.OT[m], p.K[m], SG_KS);
     pr.xh[m] = xh; pr.raw[m] = raw;
     pr.out[m] = p.out[m]; pr.K[m] = p.K[m]; pr.OT[m] = p.OT[m]; pr.NG[m] = p.NG[m];
@@ -247,7 +245,7 @@ void launch_linear_multi(const MultiLinearPlan &p, const MultiLinearArgs &a, con
   }
   launch_pdl(prep_rows_multi_kernel, dim3(((p.in + 127) / 128 + 3) / 4, p.rows, p.n), dim3(128), 0, st, x, q, p.rows, p.in, p.hi,
              (float)(1.0 / sqrt((double)p.hi)));
-  launch_stream(pr, p.MT, p.lay, p.grid, status, st);
+  launch_stream<8>(pr, p.MT, p.lay, p.grid, status, st);
   launch_pdl(linear_finish_multi_kernel, dim3(((maxout + 127) / 128 + 3) / 4, p.rows, p.n), dim3(128), 0, st, q, p.rows, p.S);
 }
 
@@ -262,7 +260,7 @@ void launch_linear(const LinearPlan &p, const void *trellis, const void *suh, co
   pr.raw = raw;
   pr.in = p.in; pr.out = p.out; pr.K = p.K; pr.rows = p.rows;
   pr.IT = p.IT; pr.OT = p.OT; pr.NG = p.NG; pr.S = p.S; pr.kc = p.kc;
-  launch_stream(pr, p.MT, p.lay, p.grid, status, st);
+  launch_stream<8>(pr, p.MT, p.lay, p.grid, status, st);
   const int chunks = (p.out + 127) / 128;
   dim3 grid((chunks + 3) / 4, p.rows);
   launch_pdl(linear_finish_kernel, grid, dim3(128), 0, st, raw, (const __half *)svh, y, p.rows, p.out, p.S, p.ho,

@@ -20,7 +20,6 @@ struct MoeParams {
   int rows;           // live rows of this run
   int P;              // rows * topk
   int has_shared;
-  int dup;            // store_a's pair form: the product mode in force when the call was enqueued
   int shared_pre;     // the shared expert's output is already in `sho` (8-bit affine shared expert: computed by other kernels)
   // weights
   const uint16_t *router;  // bf16 [E][H]
@@ -32,10 +31,10 @@ struct MoeParams {
   float *logits;           // [rows][E + 1]
   uint32_t *route;         // [rows][2 topk]
   int *plan;               // see PlanView
-  __half *xh_gu;           // [P][2][2H]  prepared gate | up operands per (row, slot) pair (store_a layout)
-  __half *xh_sgu;          // [rows][2][2H]  the shared expert's
-  __half *xh_d;            // [P][2I]  prepared down operand per pair
-  __half *xh_sd;           // [rows][2I]
+  __half *xh_gu;           // [P][2][H]  prepared gate | up operands per (row, slot) pair
+  __half *xh_sgu;          // [rows][2][H]  the shared expert's
+  __half *xh_d;            // [P][I]  prepared down operand per pair
+  __half *xh_sd;           // [rows][I]
   float *raw_gu;           // [S_gu][P][2][I]
   float *raw_sgu;          // [S_gu][rows][2][I]
   float *raw_d;            // [S_d][P][H]

@@ -24,23 +24,27 @@ static void launch_stream_ex(const P &prob, const StreamLayout &lay, int grid, i
   IJ_CUDA(cudaFuncSetAttribute(stream_gemm_kernel<P, MT, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
   launch_pdl(stream_gemm_kernel<P, MT, EX>, dim3(grid), dim3(SG_THREADS), lay.total(), st, prob, lay, status);
 }
-// the product mode in force (g_summand_product) picks the kernel; the prepared rows of the same call were written to match
+// the product mode in force (g_summand_product) picks the kernel
 template <class P, int MT>
 static void launch_stream_mt(const P &prob, const StreamLayout &lay, int grid, int *status, cudaStream_t st) {
   if (g_summand_product) launch_stream_ex<P, MT, false>(prob, lay, grid, status, st);
   else launch_stream_ex<P, MT, true>(prob, lay, grid, status, st);
 }
 
-template <class P>
+// MAXMT: the widest unit the problem has (8-row groups); narrower launches take the variant compiled for their width
+template <int MAXMT, class P>
 void launch_stream(const P &prob, int MT, const StreamLayout &lay, int grid, int *status, cudaStream_t st) {
   IJ_CHECK(lay.stages >= 2 && lay.stages <= 16, "bad ring depth %d", lay.stages);
-  switch (MT) {
-    case 1: launch_stream_mt<P, 1>(prob, lay, grid, status, st); break;
-    case 2: launch_stream_mt<P, 2>(prob, lay, grid, status, st); break;
-    case 4: launch_stream_mt<P, 4>(prob, lay, grid, status, st); break;
-    case 8: launch_stream_mt<P, 8>(prob, lay, grid, status, st); break;
-    default: fail("unsupported row tile count %d", MT);
+  IJ_CHECK(MT <= MAXMT, "unsupported row tile count %d", MT);
+  if (MT == 1) return launch_stream_mt<P, 1>(prob, lay, grid, status, st);
+  if constexpr (MAXMT >= 8) {
+    switch (MT) {
+      case 2: return launch_stream_mt<P, 2>(prob, lay, grid, status, st);
+      case 4: return launch_stream_mt<P, 4>(prob, lay, grid, status, st);
+      case 8: return launch_stream_mt<P, 8>(prob, lay, grid, status, st);
+    }
   }
+  fail("unsupported row tile count %d", MT);
 }
 
 }  // namespace ijah

@@ -11,8 +11,8 @@
 // stays busy and the consumers never wait for an operand that could have been fetched earlier. The producer warp shares
 // its scheduler with consumer warps that are always ready to issue, so every instruction it needs per stage delays the
 // stream: one copy instruction per stage (instead of one per k-tile) is what keeps the ring full. Each consumer warp owns one output tile:
-// per k-tile it reads its lane window (3 words) from the ring, decodes 8 weights per lane and issues two
-// mma.m16n8k16 per 16 activation rows; accumulators are fp32 registers. Only compressed bytes cross HBM.
+// per k-tile it reads its lane window (3 words) from the ring, decodes 8 weights per lane, rounds them with two
+// constant-matrix MMAs and issues one mma.m16n8k16 per 8 activation rows; accumulators are fp32 registers. Only compressed bytes cross HBM.
 //
 // The "problem" type P supplies the unit list and the operand / result addresses:
 //   bool P::units_final() const                        // the unit list does not depend on the preceding kernel's output
@@ -28,12 +28,6 @@
 
 #include "exl3_decode.cuh"
 #include "pipeline.cuh"
-
-// SG_DBG: timing-only builds that answer "is it the decode, the MMA or the bytes" (results are wrong on purpose):
-// 1 = decode but no MMA, 2 = MMA on the undecoded words. 0 = the product.
-#ifndef SG_DBG
-#define SG_DBG 0
-#endif
 
 namespace ijah {
 
@@ -71,14 +65,13 @@ struct UnitDesc {
 struct StreamLayout {  // dynamic shared memory carve-up (host computes, kernel mirrors)
   int stages;          // ring stages
   int stage_bytes;     // SG_KS * 8 * 32 * Kmax
-  int lda;             // A row stride in halfs (32 per k-tile + 8 pad: keeps ldmatrix rows on distinct banks)
+  int lda;             // A row stride in halfs (16 per k-tile + 8 pad: keeps ldmatrix rows on distinct banks)
   int arows;           // rows per A slot
   int aslots;          // A slots (units the producer may run ahead)
   __host__ __device__ size_t ring_off() const { return 512 + SG_MAX_ASLOTS * SG_DESC_BYTES; }
   __host__ __device__ size_t slot_bytes() const { return (size_t)arows * lda * 2; }
   __host__ __device__ size_t a_off() const { return ring_off() + (size_t)stages * stage_bytes; }
-  __host__ __device__ size_t zero_off() const { return a_off() + (size_t)aslots * slot_bytes(); }
-  __host__ __device__ size_t total() const { return zero_off() + (size_t)lda * 2; }
+  __host__ __device__ size_t total() const { return a_off() + (size_t)aslots * slot_bytes() + 64; }  // (the last row's fragment load may cover one k-tile more)
 };
 
 // shared-memory loads with the constant part of the address as an immediate (no address arithmetic per tile)
@@ -95,111 +88,105 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
                : "r"(addr), "n"(OFF));
 }
 
-// k-tile I of a stage for one output tile. The tensor core computes D^T = W'^T * X^T: the decoded tile is the A operand
-// (16 output columns x 16 k), the activations are the B operand (16 k x 8 rows). Each decoded weight arrives as the pair of
-// fp16 summands (lo, hi) the codebook function yields (dec8_raw) and takes the place of TWO k elements of the A fragment,
-// against activation rows that hold two halfs per input (store_a), so the 16 inputs of the k-tile take two mma.m16n8k16
-// per 8 activation rows: the even inputs (slots 0, 4, 2, 6 of the lane) and the odd ones (slots 1, 5, 3, 7).
-//   EX (default): one half add turns (lo, hi) into (w, w), w = fp16(lo + hi), the weight as the format defines it; the
-//                 rows hold (v, 0) and the accumulator receives w * v.
-//   !EX (opt-in): (lo, hi) goes in as it is against (v, v): lo * v + hi * v, the sum of the summands unrounded.
+// Two k-tiles (I and I + 1 of a stage) for one output tile. The tensor core computes D^T = W'^T * X^T: the decoded tile is the
+// A operand (16 output columns x 16 k), the activations are the B operand (16 k x 8 rows), one ldmatrix.x4 for both k-tiles.
+// The codebook function yields every weight as a pair of fp16 summands (lo, hi) in one register (dec8_raw).
+//   EX (default): two constant-matrix MMAs per tile (round_pairs) round and pack the lane's 8 pairs into the tile's A fragment of
+//                 fp16(lo + hi), the weights as the format defines them; one MMA per 8 rows multiplies them.
+//   !EX (opt-in): the pairs are multiplied as they are: a pair takes the place of two k elements, against (v, v) made from
+//                 the activation fragment, so a tile takes two MMAs (even inputs: slots 0, 4, 2, 6; odd: 1, 5, 3, 7) and the
+//                 accumulator receives lo * v + hi * v, the sum of the summands unrounded.
 // MT = number of 8-row groups (1, 2, 4, 8); a_row[g] is the ldmatrix address of row group g for k-tile 0 of the stage,
-// tile I sits I * 64 bytes further in the A rows. acc[g] = D^T fragment of group g: (column gq, rows 2q, 2q+1), (column gq + 8, ..).
-constexpr uint32_t SG_A_TILE_BYTES = 16 * A_HALFS_PER_INPUT * 2;  // one k-tile of one prepared activation row
+// tile I sits I * 32 bytes further in the A rows. acc[g] = D^T fragment of group g: (column gq, rows 2q, 2q+1), (column gq + 8, ..).
+// The loop is bound by instruction issue and the half-rate integer pipe, the tensor pipe has room (35 % busy): K5, block of 64
+// rows, gate / up launch: one half add per weight and (w, w) against (v, 0) pairs in doubled activation rows took 54.8
+// instructions per tile and 340 us, rounding on the tensor core takes 44.7 and 301 us (both under ncu).
+constexpr uint32_t SG_A_TILE_BYTES = 16 * 2;  // one k-tile of one prepared activation row
+
+// (v, v) of both halves of an activation fragment register
+__device__ __forceinline__ uint32_t dup_lo(uint32_t v) { return __byte_perm(v, 0u, 0x1010); }
+__device__ __forceinline__ uint32_t dup_hi(uint32_t v) { return __byte_perm(v, 0u, 0x3232); }
+
+template <bool EX>
+__device__ __forceinline__ void tile_frag(const uint32_t (&r)[8], const PairSum &ps, uint32_t (&f)[EX ? 4 : 8]) {
+  if constexpr (EX) {
+    uint32_t lo[2], hi[2];  // k 0-7 and k 8-15 of the fragment
+    round_pairs(lo, r[0], r[4], r[1], r[5], ps);
+    round_pairs(hi, r[2], r[6], r[3], r[7], ps);
+    f[0] = lo[0]; f[1] = lo[1]; f[2] = hi[0]; f[3] = hi[1];
+  } else {
+    f[0] = r[0]; f[1] = r[4]; f[2] = r[2]; f[3] = r[6];
+    f[4] = r[1]; f[5] = r[5]; f[6] = r[3]; f[7] = r[7];
+  }
+}
+template <bool EX>
+__device__ __forceinline__ void tile_mma(float (&acc)[4], const uint32_t (&f)[EX ? 4 : 8], uint32_t x0, uint32_t x1) {
+  if constexpr (EX) {
+    mma_16816(acc, f, x0, x1);
+  } else {
+    const uint32_t even[4] = {f[0], f[1], f[2], f[3]}, odd[4] = {f[4], f[5], f[6], f[7]};
+    mma_16816(acc, even, dup_lo(x0), dup_lo(x1));
+    mma_16816(acc, odd, dup_hi(x0), dup_hi(x1));
+  }
+}
 
 template <int K, bool EX, int MT, int I>
-__device__ __forceinline__ void tile_mma(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t la, const McgConst &mc,
+__device__ __forceinline__ void pair_mma(const uint32_t (&wa)[3], const uint32_t (&wb)[3], uint32_t la, const McgConst &mc, const PairSum &ps,
                                          const uint32_t (&a_row)[MT], float (&acc)[MT][4]) {
-  uint32_t r[8];
-#if SG_DBG == 2  // timing only: no decode, the raw words go to the tensor core
-  r[0] = w0; r[1] = w1; r[2] = w2; r[3] = w0 ^ la; r[4] = w1 ^ la; r[5] = w2 ^ la; r[6] = w0 + la; r[7] = w1 + la;
-#else
-  dec8_raw<K>(w0, w1, w2, la, mc, r);
-#endif
-  if constexpr (EX) {  // both halves = fp16(lo + hi), the format's weight; the activation rows then hold (v, 0) pairs
-#pragma unroll
-    for (int t = 0; t < 8; t++) {
-      const __half2 h = *reinterpret_cast<const __half2 *>(&r[t]);
-      const __half2 w = __hadd2(__low2half2(h), __high2half2(h));
-      r[t] = *reinterpret_cast<const uint32_t *>(&w);
-    }
-  }
-#if SG_DBG == 1  // timing only: decode without the MMA
-  acc[0][0] = __uint_as_float(__float_as_uint(acc[0][0]) ^ r[0] ^ r[1] ^ r[2] ^ r[3]);
-  acc[0][1] = __uint_as_float(__float_as_uint(acc[0][1]) ^ r[4] ^ r[5] ^ r[6] ^ r[7]);
-  (void)a_row;
-#else
-  const uint32_t we[4] = {r[0], r[4], r[2], r[6]}, wo[4] = {r[1], r[5], r[3], r[7]};
+  uint32_t r[8], fa[EX ? 4 : 8], fb[EX ? 4 : 8];
+  dec8_raw<K>(wa[0], wa[1], wa[2], la, mc, r);
+  tile_frag<EX>(r, ps, fa);
+  dec8_raw<K>(wb[0], wb[1], wb[2], la, mc, r);
+  tile_frag<EX>(r, ps, fb);
 #pragma unroll
   for (int g = 0; g < MT; g++) {
     uint32_t x[4];
     ldsm4<I * (int)SG_A_TILE_BYTES>(x, a_row[g]);
-    mma_16816(acc[g], we, x[0], x[1]);
-    mma_16816(acc[g], wo, x[2], x[3]);
+    tile_mma<EX>(acc[g], fa, x[0], x[1]);
+    tile_mma<EX>(acc[g], fb, x[2], x[3]);
   }
-#endif
 }
-// Half a stage (SG_HALF k-tiles starting at tile B): all window words are loaded first (3 * SG_HALF independent shared
-// loads in flight), then decoded and multiplied tile by tile. Half stages keep the window words at 12 registers; the other
-// warps of the SM cover the shared-memory latency at the start of each half.
+// Groups of SG_HALF k-tiles starting at tile B: all window words are loaded first (3 * SG_HALF independent shared loads in
+// flight), then decoded and multiplied in pairs of tiles. Groups keep the window words at 12 registers; the other warps of
+// the SM cover the shared-memory latency at the start of each group.
 constexpr int SG_HALF = 4;
 constexpr int SG_GROUPS = SG_KS / SG_HALF;
-template <int K, bool EX, int MT, int B, int I, int N>
-struct TileLoop {
-  static constexpr int KSTEP = SG_WARPS * Codec<K>::TILE_BYTES;
-  static constexpr int NP = MT;
-  static __device__ __forceinline__ void load(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t (&w)[SG_HALF][3]) {
-    w[I][0] = lds32<(B + I) * KSTEP>(p0);
-    w[I][1] = lds32<(B + I) * KSTEP>(p1);
-    w[I][2] = lds32<(B + I) * KSTEP>(p2);
-    TileLoop<K, EX, MT, B, I + 1, N>::load(p0, p1, p2, w);
-  }
-  static __device__ __forceinline__ void run(const uint32_t (&w)[SG_HALF][3], uint32_t la, const McgConst &mc, const uint32_t (&a_row)[NP],
-                                             float (&acc)[MT][4], int n) {
-    if (B + I < n) tile_mma<K, EX, MT, B + I>(w[I][0], w[I][1], w[I][2], la, mc, a_row, acc);
-    TileLoop<K, EX, MT, B, I + 1, N>::run(w, la, mc, a_row, acc, n);
-  }
-  static __device__ __forceinline__ void run_all(const uint32_t (&w)[SG_HALF][3], uint32_t la, const McgConst &mc, const uint32_t (&a_row)[NP],
-                                                 float (&acc)[MT][4]) {  // straight-line: the tiles interleave freely
-    tile_mma<K, EX, MT, B + I>(w[I][0], w[I][1], w[I][2], la, mc, a_row, acc);
-    TileLoop<K, EX, MT, B, I + 1, N>::run_all(w, la, mc, a_row, acc);
-  }
-};
-template <int K, bool EX, int MT, int B, int N>
-struct TileLoop<K, EX, MT, B, N, N> {
-  static constexpr int NP = MT;
-  static __device__ __forceinline__ void load(uint32_t, uint32_t, uint32_t, uint32_t (&)[SG_HALF][3]) {}
-  static __device__ __forceinline__ void run(const uint32_t (&)[SG_HALF][3], uint32_t, const McgConst &, const uint32_t (&)[NP], float (&)[MT][4], int) {}
-  static __device__ __forceinline__ void run_all(const uint32_t (&)[SG_HALF][3], uint32_t, const McgConst &, const uint32_t (&)[NP], float (&)[MT][4]) {}
-};
 
-// the SG_GROUPS groups of a stage, one after the other
-template <int K, bool EX, int MT, int G, int NG>
-struct StageLoop {
-  static constexpr int NP = MT;
-  static __device__ __forceinline__ void run_all(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t (&w)[SG_HALF][3], uint32_t la, const McgConst &mc,
-                                                 const uint32_t (&a_row)[NP], float (&acc)[MT][4]) {
-    TileLoop<K, EX, MT, G * SG_HALF, 0, SG_HALF>::load(p0, p1, p2, w);
-    TileLoop<K, EX, MT, G * SG_HALF, 0, SG_HALF>::run_all(w, la, mc, a_row, acc);
-    StageLoop<K, EX, MT, G + 1, NG>::run_all(p0, p1, p2, w, la, mc, a_row, acc);
+// the groups G .. of a full stage, one after the other
+template <int K, bool EX, int MT, int G>
+__device__ __forceinline__ void stage_groups(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t la, const McgConst &mc, const PairSum &ps,
+                                             const uint32_t (&a_row)[MT], float (&acc)[MT][4]) {
+  if constexpr (G < SG_GROUPS) {
+    constexpr int B = G * SG_HALF, KSTEP = SG_WARPS * Codec<K>::TILE_BYTES;
+    static_assert(SG_HALF == 4, "two pairs of tiles per group");
+    uint32_t w[SG_HALF][3];
+    w[0][0] = lds32<(B + 0) * KSTEP>(p0); w[0][1] = lds32<(B + 0) * KSTEP>(p1); w[0][2] = lds32<(B + 0) * KSTEP>(p2);
+    w[1][0] = lds32<(B + 1) * KSTEP>(p0); w[1][1] = lds32<(B + 1) * KSTEP>(p1); w[1][2] = lds32<(B + 1) * KSTEP>(p2);
+    w[2][0] = lds32<(B + 2) * KSTEP>(p0); w[2][1] = lds32<(B + 2) * KSTEP>(p1); w[2][2] = lds32<(B + 2) * KSTEP>(p2);
+    w[3][0] = lds32<(B + 3) * KSTEP>(p0); w[3][1] = lds32<(B + 3) * KSTEP>(p1); w[3][2] = lds32<(B + 3) * KSTEP>(p2);
+    pair_mma<K, EX, MT, B>(w[0], w[1], la, mc, ps, a_row, acc);
+    pair_mma<K, EX, MT, B + 2>(w[2], w[3], la, mc, ps, a_row, acc);
+    stage_groups<K, EX, MT, G + 1>(p0, p1, p2, la, mc, ps, a_row, acc);
   }
-  static __device__ __forceinline__ void run(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t (&w)[SG_HALF][3], uint32_t la, const McgConst &mc,
-                                             const uint32_t (&a_row)[NP], float (&acc)[MT][4], int n) {
-    if (G * SG_HALF < n) {
-      TileLoop<K, EX, MT, G * SG_HALF, 0, SG_HALF>::load(p0, p1, p2, w);
-      TileLoop<K, EX, MT, G * SG_HALF, 0, SG_HALF>::run(w, la, mc, a_row, acc, n);
+}
+// the n < SG_KS tiles of a short last stage, one at a time
+template <int K, bool EX, int MT>
+__device__ __forceinline__ void stage_tail(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t la, const McgConst &mc, const PairSum &ps,
+                                           const uint32_t (&a_row)[MT], float (&acc)[MT][4], int n) {
+  constexpr uint32_t KSTEP = SG_WARPS * Codec<K>::TILE_BYTES;
+#pragma unroll 1
+  for (int i = 0; i < n; i++) {
+    uint32_t r[8], f[EX ? 4 : 8];
+    dec8_raw<K>(lds32<0>(p0 + i * KSTEP), lds32<0>(p1 + i * KSTEP), lds32<0>(p2 + i * KSTEP), la, mc, r);
+    tile_frag<EX>(r, ps, f);
+#pragma unroll
+    for (int g = 0; g < MT; g++) {
+      uint32_t x[4];
+      ldsm4<0>(x, a_row[g] + i * SG_A_TILE_BYTES);
+      tile_mma<EX>(acc[g], f, x[0], x[1]);
     }
-    StageLoop<K, EX, MT, G + 1, NG>::run(p0, p1, p2, w, la, mc, a_row, acc, n);
   }
-};
-template <int K, bool EX, int MT, int NG>
-struct StageLoop<K, EX, MT, NG, NG> {
-  static constexpr int NP = MT;
-  static __device__ __forceinline__ void run_all(uint32_t, uint32_t, uint32_t, uint32_t (&)[SG_HALF][3], uint32_t, const McgConst &,
-                                                 const uint32_t (&)[NP], float (&)[MT][4]) {}
-  static __device__ __forceinline__ void run(uint32_t, uint32_t, uint32_t, uint32_t (&)[SG_HALF][3], uint32_t, const McgConst &,
-                                             const uint32_t (&)[NP], float (&)[MT][4], int) {}
-};
+}
 
 // The consumer side of the ring, all in registers: stage index and parity, the shared-memory addresses of the barriers
 // (empty[s] sits SG_MAX_STAGES * 8 bytes after full[s]) and of the warp's tile inside stage 0.
@@ -221,8 +208,8 @@ constexpr uint32_t SG_EMPTY_OFF = SG_MAX_STAGES * 8;
 // straight-line code between one wait and one arrive; a short last stage and the warps without a tile (units narrower
 // than 8 tiles) take their own loops.
 template <int K, bool EX, int MT>
-__device__ __forceinline__ bool consume_unit(const UnitDesc &d, RingCursor &rc, bool live, int lane, const McgConst &mc, uint32_t a_addr,
-                                             uint32_t lda_bytes, uint32_t z_addr, const int *rowoff, int col, int *status) {
+__device__ __forceinline__ bool consume_unit(const UnitDesc &d, RingCursor &rc, bool live, int lane, const McgConst &mc, const PairSum &ps, uint32_t a_addr,
+                                             uint32_t lda_bytes, const int *rowoff, int col, int *status) {
   const uint32_t lane0 = lane == 0 ? 1u : 0u;
   const int nfull = d.kc / SG_KS, rem = d.kc - nfull * SG_KS;
   if (!live) {
@@ -239,8 +226,7 @@ __device__ __forceinline__ bool consume_unit(const UnitDesc &d, RingCursor &rc, 
   for (int m = 0; m < MT; m++)
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[m][j] = 0.0f;
-  // ldmatrix.x4 row addresses of an 8-row group: lanes 8j .. 8j+7 give rows 0-7 at byte 16 j of the k-tile (the even
-  // inputs' low and high halves of the tile, then the odd inputs'). A dead row (its results are never stored) reads the
+  // ldmatrix.x4 row addresses of an 8-row group: lanes 8j .. 8j+7 give rows 0-7 at byte 16 j of a pair of k-tiles. A dead row (its results are never stored) reads the
   // unit's row 0 again: the same address as a live lane, i.e. a broadcast. (A separate zero row sat at the same offset
   // modulo 128 bytes as row 0 and cost every ldmatrix a two-way bank conflict: 4 of 14 load wavefronts per tile.)
   uint32_t a_row[MT];
@@ -252,26 +238,24 @@ __device__ __forceinline__ bool consume_unit(const UnitDesc &d, RingCursor &rc, 
       a_row[m] = a_addr + (uint32_t)(r < d.nrows ? r : 0) * lda_bytes + lkof;
     }
   }
-  (void)z_addr;
   const typename Codec<K>::Lane L = Codec<K>::lane(lane);
   const uint32_t d1 = L.o1 - L.o0, d2 = L.o2 - L.o0, t0 = rc.tile0 + L.o0;
-  uint32_t w[SG_HALF][3];
   for (int s = 0; s < nfull; s++) {
     const uint32_t bar = rc.full + rc.stage * 8u;
     if (!mbar_wait_poll(bar, rc.phase)) { atomicExch(status, 2); return false; }
     const uint32_t p0 = t0 + rc.stage * rc.stage_bytes, p1 = p0 + d1, p2 = p0 + d2;
-    StageLoop<K, EX, MT, 0, SG_GROUPS>::run_all(p0, p1, p2, w, L.a, mc, a_row, acc);
+    stage_groups<K, EX, MT, 0>(p0, p1, p2, L.a, mc, ps, a_row, acc);
 #pragma unroll
-    for (int m = 0; m < MT; m++) a_row[m] += SG_KS * SG_A_TILE_BYTES;  // the zero row is a full row too
+    for (int m = 0; m < MT; m++) a_row[m] += SG_KS * SG_A_TILE_BYTES;
     __syncwarp();
     mbar_arrive_if(bar + SG_EMPTY_OFF, lane0);
     rc.advance();
   }
-  if (rem) {  // a short last stage: the loads beyond it read stale ring bytes that are never used
+  if (rem) {  // a short last stage
     const uint32_t bar = rc.full + rc.stage * 8u;
     if (!mbar_wait_poll(bar, rc.phase)) { atomicExch(status, 2); return false; }
     const uint32_t p0 = t0 + rc.stage * rc.stage_bytes, p1 = p0 + d1, p2 = p0 + d2;
-    StageLoop<K, EX, MT, 0, SG_GROUPS>::run(p0, p1, p2, w, L.a, mc, a_row, acc, rem);
+    stage_tail<K, EX, MT>(p0, p1, p2, L.a, mc, ps, a_row, acc, rem);
     __syncwarp();
     mbar_arrive_if(bar + SG_EMPTY_OFF, lane0);
     rc.advance();
@@ -294,28 +278,14 @@ __device__ __forceinline__ bool consume_unit(const UnitDesc &d, RingCursor &rc, 
   return true;
 }
 
-// per-unit dispatch on the unit's live rows: a launch compiled for up to 8 * MT rows runs a unit with fewer rows through the
-// narrowest path that holds them (one MMA per 8 rows), since most units of a wide launch are experts that only one or two
-// rows selected
-template <int K, bool EX, int MT, int SUB>
-__device__ __forceinline__ bool consume_rows(const UnitDesc &d, RingCursor &rc, bool live, int lane, const McgConst &mc, uint32_t a_addr,
-                                             uint32_t lda_bytes, uint32_t z_addr, const int *rowoff, int col, int *status) {
-  if constexpr (SUB < MT) {
-    if (d.nrows <= 8 * SUB) return consume_unit<K, EX, SUB>(d, rc, live, lane, mc, a_addr, lda_bytes, z_addr, rowoff, col, status);
-    return consume_rows<K, EX, MT, SUB * 2>(d, rc, live, lane, mc, a_addr, lda_bytes, z_addr, rowoff, col, status);
-  } else {
-    return consume_unit<K, EX, MT>(d, rc, live, lane, mc, a_addr, lda_bytes, z_addr, rowoff, col, status);
-  }
-}
-
 template <bool EX, int MT>
-__device__ __forceinline__ bool consume_any(const UnitDesc &d, RingCursor &rc, bool live, int warp, int lane, const McgConst &mc, uint32_t a_addr,
-                                            uint32_t lda_bytes, uint32_t z_addr, const int *rowoff, int col, int *status) {
+__device__ __forceinline__ bool consume_any(const UnitDesc &d, RingCursor &rc, bool live, int warp, int lane, const McgConst &mc, const PairSum &ps, uint32_t a_addr,
+                                            uint32_t lda_bytes, const int *rowoff, int col, int *status) {
   const uint32_t ring0 = rc.tile0;  // address of stage 0; the warp's tile offset depends on the unit's K
 #define SG_CASE(KK)                                                                                              \
   case KK: {                                                                                                     \
     rc.tile0 = ring0 + (uint32_t)warp * Codec<KK>::TILE_BYTES;                                                   \
-    const bool ok = consume_rows<KK, EX, MT, 1>(d, rc, live, lane, mc, a_addr, lda_bytes, z_addr, rowoff, col, status); \
+    const bool ok = consume_unit<KK, EX, MT>(d, rc, live, lane, mc, ps, a_addr, lda_bytes, rowoff, col, status); \
     rc.tile0 = ring0;                                                                                            \
     return ok;                                                                                                   \
   }
@@ -341,7 +311,6 @@ __global__ void __launch_bounds__(SG_THREADS, SG_CTAS) stream_gemm_kernel(const 
   unsigned char *desc = smem + 512;  // per A slot: the unit descriptor, then the output row offsets of its rows
   unsigned char *ring = smem + lay.ring_off();
   unsigned char *aslot = smem + lay.a_off();
-  unsigned char *zrow = smem + lay.zero_off();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -355,7 +324,6 @@ __global__ void __launch_bounds__(SG_THREADS, SG_CTAS) stream_gemm_kernel(const 
     }
     mbar_fence_init();
   }
-  for (int i = threadIdx.x; i < lay.lda / 2; i += blockDim.x) reinterpret_cast<uint32_t *>(zrow)[i] = 0u;
   __syncthreads();
 
   if (warp == SG_WARPS) {
@@ -451,9 +419,10 @@ __global__ void __launch_bounds__(SG_THREADS, SG_CTAS) stream_gemm_kernel(const 
   rc.stage_bytes = (uint32_t)lay.stage_bytes; rc.nstages = (uint32_t)lay.stages; rc.stage = 0u; rc.phase = 0u;
   int slot = 0;
   uint32_t aphase = 0;
-  const uint32_t a0_addr = smem_u32(aslot), z_addr = smem_u32(zrow), slot_bytes = (uint32_t)lay.slot_bytes(), lda_bytes = (uint32_t)lay.lda * 2u;
+  const uint32_t a0_addr = smem_u32(aslot), slot_bytes = (uint32_t)lay.slot_bytes(), lda_bytes = (uint32_t)lay.lda * 2u;
   const uint32_t afull_a = smem_u32(a_full), aempty_a = smem_u32(a_empty);
   const McgConst mc = McgConst::load();
+  const PairSum ps = PairSum::make(lane);
   const int col = warp * 16 + (lane >> 2);
 
   if (!prob.units_final()) pdl_wait();  // the unit count is the predecessor's output
@@ -462,7 +431,7 @@ __global__ void __launch_bounds__(SG_THREADS, SG_CTAS) stream_gemm_kernel(const 
     if (!mbar_wait_a(afull_a + (uint32_t)slot * 8u, aphase, status, 4)) return;
     const UnitDesc d = *reinterpret_cast<const UnitDesc *>(desc + (size_t)slot * SG_DESC_BYTES);
     const int *rowoff = reinterpret_cast<const int *>(desc + (size_t)slot * SG_DESC_BYTES + SG_DESC_UNIT_BYTES);
-    if (!consume_any<EX, MT>(d, rc, warp < d.ntiles, warp, lane, mc, a0_addr + (uint32_t)slot * slot_bytes, lda_bytes, z_addr, rowoff, col, status))
+    if (!consume_any<EX, MT>(d, rc, warp < d.ntiles, warp, lane, mc, ps, a0_addr + (uint32_t)slot * slot_bytes, lda_bytes, rowoff, col, status))
       return;
     // the stores above read the slot's row offsets: only now may it be refilled
     __syncwarp();

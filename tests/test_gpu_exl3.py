@@ -79,6 +79,32 @@ def test_linear_matches_oracle(eng, n_in, n_out, K, rows):
     assert np.array_equal(y, yh)
 
 
+@pytest.mark.parametrize("K", [4, 5, 6, 7, 8])
+@pytest.mark.parametrize("n_in", [128, 64 * 5 + 16])  # whole ring stages, and a short last stage (21 k-tiles, Hadamard 16)
+def test_stream_product_uses_the_rounded_weights(eng, K, n_in):
+    # rows that prepare to unit vectors read single weights out of the stream kernel: y[i] = H(W'[i]) for 64 rows i. The sums
+    # before the output transform have one non-zero term, so only its f32 butterflies round: at most 8 roundings of partial
+    # sums below sqrt(128) times the largest |W'| (4), i.e. 8 * 2^-24 * 4; an unrounded weight would be off by 2^-12.
+    import torch
+    from ijah_b200 import engine as E
+    rng = np.random.default_rng(70 + K)
+    tr, _, _ = packgen.exl3_linear(rng, n_in, 2048, K)
+    lin = E.Exl3Linear(eng, tr, np.ones(n_in, np.float16), np.ones(2048, np.float16))
+
+    def had(n):
+        h = np.ones((1, 1))
+        while h.shape[0] < n:
+            h = np.block([[h, h], [h, -h]])
+        return h / np.sqrt(n)
+    hn = next(n for n in (128, 64, 32, 16) if n_in % n == 0)
+    x = np.kron(np.eye(n_in // hn), had(hn))[-64:].astype(np.float32)  # the last 64 unit vectors, transformed
+    y = lin(torch.from_numpy(x).cuda()).cpu().numpy()
+    w = CO.decode_inner(tr)[-64:].astype(np.float64)
+    want = (w.reshape(64, -1, 128) @ had(128)).reshape(64, -1)
+    assert np.abs(y - want).max() < 2e-6
+    assert eng.lib.ne_device_wait_status() == 0
+
+
 def test_trunk_fixture_from_reference(eng):
     import torch
     from ijah_b200 import engine as E
