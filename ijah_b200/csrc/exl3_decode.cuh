@@ -201,25 +201,46 @@ __device__ __forceinline__ void fwht_chunk(float (&v)[4], int lane, int N, float
   for (int j = 0; j < 4; j++) v[j] *= scale;
 }
 
-// The same transform of size 128 with the chunk held as (4 lane .. 4 lane + 3) per lane, so that a lane reads and writes 16
-// contiguous bytes. Same butterflies in the same order (index bits 0, 1 inside the lane, bits 2..6 across lanes), hence
-// bit-identical to fwht_chunk.
-__device__ __forceinline__ void fwht128_contig(float (&v)[4], int lane, float scale) {
-  {
-    const float a = v[0] + v[1], b = v[0] - v[1], c = v[2] + v[3], d = v[2] - v[3];
-    v[0] = a + c; v[1] = b + d; v[2] = a - c; v[3] = b - d;
+// The same transform of size 128 with a chunk held by FOUR lanes, 32 elements each, so that a warp transforms eight chunks at
+// once (all 32 lanes call; l = lane & 3). In: v[4 i + j] = element 16 i + 4 l + j (a lane loads 16 contiguous bytes, four lanes
+// 64). Out: v[8 t' + ..] = 32 CONTIGUOUS elements, those from quad_first(lane) on.
+// What bounds a transform here is the shuffle pipe (16 lanes per clock per SM): with a chunk spread over 32 lanes it takes 20
+// shuffles, in this form 4. Index bits 0, 1, 4, 5, 6 are butterflies inside the lane. Bits 2 and 3 are exchanges: a lane gives
+// the half of its elements that its partner keeps and gets the partner's other half, then adds and subtracts in its own
+// registers, one shuffle per two elements. The difference comes out negated in the upper lane of a pair; nothing mixes it with
+// elements of the other sign afterwards, so the sign is put right in the final multiply.
+__device__ __forceinline__ int quad_first(int lane) { return (lane & 1) * 64 + ((lane >> 1) & 1) * 32; }
+__device__ __forceinline__ void fwht128_quad(float (&v)[32], int lane, float scale) {
+#pragma unroll
+  for (int st = 1; st < 32; st <<= 1)
+#pragma unroll
+    for (int p = 0; p < 32; p++)
+      if ((p & st) == 0) {
+        const float a = v[p] + v[p + st], b = v[p] - v[p + st];
+        v[p] = a; v[p + st] = b;
+      }
+  const bool up1 = lane & 1, up2 = lane & 2;
+#pragma unroll
+  for (int p = 0; p < 16; p++) {  // bit 2, exchanged with bit 6
+    const float keep = up1 ? v[p + 16] : v[p], got = __shfl_xor_sync(0xFFFFFFFFu, up1 ? v[p] : v[p + 16], 1);
+    v[p] = keep + got; v[p + 16] = keep - got;
   }
 #pragma unroll
-  for (int bit = 1; bit < 32; bit <<= 1) {
-    const float sgn = (lane & bit) == 0 ? 1.0f : -1.0f;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const float p = __shfl_xor_sync(0xFFFFFFFFu, v[j], bit);
-      v[j] = __fmaf_rn(v[j], sgn, p);
+  for (int p = 0; p < 32; p++)
+    if ((p & 8) == 0) {  // bit 3, exchanged with bit 5
+      const float keep = up2 ? v[p + 8] : v[p], got = __shfl_xor_sync(0xFFFFFFFFu, up2 ? v[p] : v[p + 8], 2);
+      v[p] = keep + got; v[p + 8] = keep - got;
     }
+  // now v[16 h + 8 t + 4 i + j] is element quad_first + 16 i + 8 t + 4 h + j
+  const float s1 = up1 ? -scale : scale, s2 = up2 ? -scale : scale, s12 = up1 != up2 ? -scale : scale;
+  float o[32];
+#pragma unroll
+  for (int p = 0; p < 32; p++) {
+    const int h = p >> 4, t = (p >> 3) & 1, i = (p >> 2) & 1, j = p & 3;
+    o[16 * i + 8 * t + 4 * h + j] = v[p] * (h ? (t ? s12 : s1) : (t ? s2 : scale));
   }
 #pragma unroll
-  for (int j = 0; j < 4; j++) v[j] *= scale;
+  for (int p = 0; p < 32; p++) v[p] = o[p];
 }
 
 __host__ __device__ inline int had_size(int d) { return d % 128 == 0 ? 128 : d % 64 == 0 ? 64 : d % 32 == 0 ? 32 : 16; }

@@ -4,6 +4,7 @@
 #include "common.hpp"
 #include "exl3_decode.cuh"
 #include "pf_moe.cuh"
+#include "stream_gemm.cuh"
 #include "umma.cuh"
 
 namespace ijah {
@@ -45,27 +46,61 @@ struct PgSmem {
   uint32_t tmem_base;
 };
 
+// A decoder warp's view of the two rings
+struct PgCursor {
+  uint32_t rs, as, rph, aph;
+};
+
+// All stages of one item for one decoder warp (column tile dw): straight-line code for one K, so that the lane's constants of
+// the other four do not compete for registers (with the choice of K inside the stage loop they spilled).
 template <int K>
-__device__ __forceinline__ void pg_decode_stage(const unsigned char *ring_stage, unsigned char *a_stage, int dw, int lane) {
+__device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, uint32_t ring_stage_bytes, uint32_t abuf, PgCursor &cu, int nst,
+                                               int dw, int lane, int *status) {
   const typename Codec<K>::Lane L = Codec<K>::lane(lane);
   const McgConst mc = McgConst::load();
-  const int ng = dw >> 3, t = dw & 7, q = lane & 3, c = lane >> 2;
+  const PairSum ps = PairSum::make(lane);
+  constexpr int KSTEP = 16 * Codec<K>::TILE_BYTES;
+  const uint32_t tile0 = ring + dw * Codec<K>::TILE_BYTES + L.o0, d1 = L.o1 - L.o0, d2 = L.o2 - L.o0;
+  // lane (q, c) = (lane & 3, lane >> 2) writes k (2q, 2q + 1) and (2q + 8, 2q + 9) of columns c and c + 8
+  const uint32_t dst0 = abuf + (uint32_t)((dw >> 3) * 4096 + (dw & 7) * 256 + lane * 4);
+  const uint32_t bars = smem_u32(sm);
+  const uint32_t rfull = bars + (uint32_t)offsetof(PgSmem, ring_full), rempty = bars + (uint32_t)offsetof(PgSmem, ring_empty);
+  const uint32_t afull = bars + (uint32_t)offsetof(PgSmem, a_full), aempty = bars + (uint32_t)offsetof(PgSmem, ab_empty);
+  const uint32_t lane0 = lane == 0 ? 1u : 0u;
+#pragma unroll 1
+  for (int st = 0; st < nst; st++) {
+    if (!mbar_wait_a(rfull + cu.rs * 8u, cu.rph, status, 17)) return false;
+    if (!mbar_wait_a(aempty + cu.as * 8u, cu.aph ^ 1u, status, 18)) return false;
+    const uint32_t p0 = tile0 + cu.rs * ring_stage_bytes, p1 = p0 + d1, p2 = p0 + d2, dst = dst0 + cu.as * (uint32_t)PG_A_STAGE;
+    static_assert(PG_KS == 4, "four k-tiles per stage");
+    uint32_t w[4][3];
+    w[0][0] = lds32<0 * KSTEP>(p0); w[0][1] = lds32<0 * KSTEP>(p1); w[0][2] = lds32<0 * KSTEP>(p2);
+    w[1][0] = lds32<1 * KSTEP>(p0); w[1][1] = lds32<1 * KSTEP>(p1); w[1][2] = lds32<1 * KSTEP>(p2);
+    w[2][0] = lds32<2 * KSTEP>(p0); w[2][1] = lds32<2 * KSTEP>(p1); w[2][2] = lds32<2 * KSTEP>(p2);
+    w[3][0] = lds32<3 * KSTEP>(p0); w[3][1] = lds32<3 * KSTEP>(p1); w[3][2] = lds32<3 * KSTEP>(p2);
 #pragma unroll
-  for (int ks = 0; ks < PG_KS; ks++) {
-    const unsigned char *tile = ring_stage + (size_t)(ks * 16 + dw) * Codec<K>::TILE_BYTES;
-    uint32_t b[4];
-    dec8<K>(*reinterpret_cast<const uint32_t *>(tile + L.o0), *reinterpret_cast<const uint32_t *>(tile + L.o1),
-            *reinterpret_cast<const uint32_t *>(tile + L.o2), L.a, mc, b);
-    // lane (q, c): b[0] = k (2q, 2q+1) of column c, b[1] = k (2q+8, 2q+9) of column c, b[2], b[3] the same of column c + 8
-    unsigned char *dst = a_stage + (size_t)(ks * 2 + ng) * 4096 + (2 * t) * 128 + c * 16 + q * 4;
-    *reinterpret_cast<uint32_t *>(dst) = b[0];
-    *reinterpret_cast<uint32_t *>(dst + 2048) = b[1];
-    *reinterpret_cast<uint32_t *>(dst + 128) = b[2];
-    *reinterpret_cast<uint32_t *>(dst + 128 + 2048) = b[3];
+    for (int ks = 0; ks < PG_KS; ks++) {
+      uint32_t r[8], lo[2], hi[2];
+      dec8_raw<K>(w[ks][0], w[ks][1], w[ks][2], L.a, mc, r);
+      round_pairs(lo, r[0], r[4], r[1], r[5], ps);
+      round_pairs(hi, r[2], r[6], r[3], r[7], ps);
+      const uint32_t d = dst + ks * 8192;  // (the offsets below are immediates)
+      asm volatile(
+          "st.shared.u32 [%0], %1;\n\tst.shared.u32 [%0+2048], %2;\n\tst.shared.u32 [%0+128], %3;\n\tst.shared.u32 [%0+2176], %4;"
+          ::"r"(d), "r"(lo[0]), "r"(hi[0]), "r"(lo[1]), "r"(hi[1])
+          : "memory");
+    }
+    fence_proxy_async_smem();  // the tensor core reads what these ordinary stores wrote
+    __syncwarp();
+    mbar_arrive_if(afull + cu.as * 8u, lane0);
+    mbar_arrive_if(rempty + cu.rs * 8u, lane0);
+    if (++cu.rs == PG_RING) { cu.rs = 0; cu.rph ^= 1u; }
+    if (++cu.as == PG_AB) { cu.as = 0; cu.aph ^= 1u; }
   }
+  return true;
 }
 
-__global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const PgGemm g, int *status) {
+__global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_constant__ PgGemm g, int *status) {
   extern __shared__ __align__(1024) unsigned char pf_smem[];
   unsigned char *smem = pf_smem;
   PgSmem *sm = reinterpret_cast<PgSmem *>(smem);
@@ -160,13 +195,20 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const PgGemm g, 
       if (!mbar_wait(&sm->acc_full[buf], cph[buf], status, 16)) break;
       tc_fence_after_sync();
       float *out = g.out[im.proj] + (size_t)im.row0 * g.ldo + im.ngpair * PF_NCOL + qd * 32 + lane;
+#pragma unroll 1
       for (int ng = 0; ng < 2; ng++)
+#pragma unroll 1
         for (int c0 = 0; c0 < im.nrows; c0 += 32) {
           uint32_t r[32];
           tmem_ld_32x32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(buf * 2 + ng) * 128u + (uint32_t)c0, r);
+          float *o = out + (size_t)c0 * g.ldo + ng * 128;
+          uint32_t ld = (uint32_t)g.ldo;
+          asm volatile("" : "+r"(ld));  // (32 precomputed row offsets would not fit the registers)
 #pragma unroll
-          for (int j = 0; j < 32; j++)
-            if (c0 + j < im.nrows) out[(size_t)(c0 + j) * g.ldo + ng * 128] = __uint_as_float(r[j]);
+          for (int j = 0; j < 32; j++) {
+            if (c0 + j < im.nrows) *o = __uint_as_float(r[j]);
+            o += ld;
+          }
         }
       tc_fence_before_sync();
       __syncwarp();
@@ -177,31 +219,20 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const PgGemm g, 
   } else {
     // ------------------------------------------------------------------------------------------ decoders
     const int dw = warp - 6;
-    int rs = 0, as = 0;
-    uint32_t rph = 0, aph = 0;
+    PgCursor cu{0u, 0u, 0u, 0u};
+    const uint32_t ring_a = smem_u32(ring), abuf_a = smem_u32(abuf);
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const PfItem im = g.items[it];
-      const int K = im.expert < 0 ? g.Ks : g.Kx;
-      for (int st = 0; st < nst; st++) {
-        if (!mbar_wait(&sm->ring_full[rs], rph, status, 17)) goto out;
-        if (!mbar_wait(&sm->ab_empty[as], aph ^ 1u, status, 18)) goto out;
-        const unsigned char *rsrc = ring + (size_t)rs * ring_stage_bytes;
-        unsigned char *adst = abuf + (size_t)as * PG_A_STAGE;
-        switch (K) {
-          case 4: pg_decode_stage<4>(rsrc, adst, dw, lane); break;
-          case 5: pg_decode_stage<5>(rsrc, adst, dw, lane); break;
-          case 6: pg_decode_stage<6>(rsrc, adst, dw, lane); break;
-          case 7: pg_decode_stage<7>(rsrc, adst, dw, lane); break;
-          default: pg_decode_stage<8>(rsrc, adst, dw, lane); break;
-        }
-        fence_proxy_async_smem();  // the tensor core reads what these ordinary stores wrote
-        __syncwarp();
-        if (lane == 0) { mbar_arrive(&sm->a_full[as]); mbar_arrive(&sm->ring_empty[rs]); }
-        if (++rs == PG_RING) { rs = 0; rph ^= 1u; }
-        if (++as == PG_AB) { as = 0; aph ^= 1u; }
+      const int K = g.items[it].expert < 0 ? g.Ks : g.Kx;
+      bool ok;
+      switch (K) {
+        case 4: ok = pg_decode_item<4>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
+        case 5: ok = pg_decode_item<5>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
+        case 6: ok = pg_decode_item<6>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
+        case 7: ok = pg_decode_item<7>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
+        default: ok = pg_decode_item<8>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
       }
+      if (!ok) break;
     }
-  out:;
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -548,185 +579,179 @@ __global__ void __launch_bounds__(32) pf_place_kernel(const PfParams p, int *ord
   }
 }
 
-// The three elementwise kernels below give one warp a whole operand row (one position, or one slot of one token): the
-// row's metadata is fetched once, the loads of several 128-element chunks are in flight together, and a lane owns 4
-// consecutive elements of a chunk, i.e. 8 bytes of fp16 output: half a row of a core matrix of the blocked layout.
-// All three are bound by instruction issue (the fp32 Hadamard butterflies and their shuffles), not by memory.
+// The elementwise kernels below give four lanes one 128-element chunk of a row (fwht128_quad) and a warp the same chunk of the
+// eight rows of one row group of the blocked layout, whose rows all belong to one expert: what the warp writes of a core matrix
+// is then 128 contiguous bytes without a detour through shared memory, and the scale vectors are one broadcast per warp.
+// Prefill of 4096 tokens, Zipf routing: with one warp per row and 20 shuffles per chunk the three were bound by the shuffle pipe.
 constexpr float PF_HS = 0.08838834764831845f;  // 1 / sqrt(128)
 
-__device__ __forceinline__ float4 mul4(float4 a, uint2 h) {  // a * (4 halfs)
-  const __half2 h0 = *reinterpret_cast<const __half2 *>(&h.x), h1 = *reinterpret_cast<const __half2 *>(&h.y);
-  const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-  return make_float4(a.x * f0.x, a.y * f0.y, a.z * f1.x, a.w * f1.y);
+// v[4 i + j] = element 16 i + 4 l + j of the lane's chunk of an f32 row
+__device__ __forceinline__ void quad_load(float (&v)[32], const float *chunk, int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const float4 a = *reinterpret_cast<const float4 *>(chunk + 16 * i + 4 * (lane & 3));
+    v[4 * i] = a.x; v[4 * i + 1] = a.y; v[4 * i + 2] = a.z; v[4 * i + 3] = a.w;
+  }
 }
-__device__ __forceinline__ uint2 pack4(const float (&v)[4]) {
-  const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
-  return make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+// v *= the halfs of a scale vector's chunk, elements in the order of quad_load
+__device__ __forceinline__ void quad_scale_in(float (&v)[32], const __half *chunk, int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const uint2 h = *reinterpret_cast<const uint2 *>(chunk + 16 * i + 4 * (lane & 3));
+    const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&h.x)), f1 = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
+    v[4 * i] *= f0.x; v[4 * i + 1] *= f0.y; v[4 * i + 2] *= f1.x; v[4 * i + 3] *= f1.y;
+  }
 }
-// lane's 4 elements (k = chunk * 128 + 4 lane ..) of position pos in a blocked operand with `in` columns
-__device__ __forceinline__ __half *blocked_lane_ptr(__half *base, int pos, int chunk, int lane, int in) {
-  return base + (((size_t)(pos >> 3) * (in >> 3) + chunk * 16 + (lane >> 1)) << 6) + ((pos & 7) << 3) + ((lane & 1) << 2);
+// v *= the halfs of a scale vector's chunk, 32 elements from quad_first(lane) on (the order after the transform)
+__device__ __forceinline__ void quad_scale_out(float (&v)[32], const __half *chunk, int lane) {
+  const uint4 *src = reinterpret_cast<const uint4 *>(chunk + quad_first(lane));
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const uint4 u = src[c];
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[j]));
+      v[8 * c + 2 * j] *= f.x; v[8 * c + 2 * j + 1] *= f.y;
+    }
+  }
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+// fp16(v) into a blocked operand with `in` columns: chunk `chunk` of position pos
+__device__ __forceinline__ void quad_store_blocked(const float (&v)[32], __half *base, int pos, int chunk, int lane, int in) {
+  __half *dst = base + (((size_t)(pos >> 3) * (in >> 3) + chunk * 16 + (quad_first(lane) >> 3)) << 6) + ((pos & 7) << 3);
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+    *reinterpret_cast<uint4 *>(dst + 64 * c) = make_uint4(pack2(v[8 * c], v[8 * c + 1]), pack2(v[8 * c + 2], v[8 * c + 3]),
+                                                         pack2(v[8 * c + 4], v[8 * c + 5]), pack2(v[8 * c + 6], v[8 * c + 7]));
+}
+__device__ __forceinline__ void quad_zero(float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; j++) v[j] = 0.0f;
 }
 
-// gate / up operands: xh[pos] = fp16(H128(x[token(pos)] * suh[expert(pos)])), one warp per position, eight positions (one
-// row group of the blocked layout) per CTA (reference kernels/prefill/pf_moe.metal:88-104); padding positions are written
-// as zeros. In the blocked layout the eight rows of a group and one 128-input chunk form 2 KB of contiguous memory (16
-// core matrices of 8 rows x 16 bytes), of which a warp (one row) owns every eighth 16 bytes: the CTA therefore collects
-// four chunks of both operands in shared memory (16-byte slots XOR-swizzled by core matrix: conflict-free both ways)
-// and writes them out as whole 512-byte runs per warp instead of 16-byte pieces.
+// gate / up operands: xh[pos] = fp16(H128(x[token(pos)] * suh[expert(pos)])) (reference kernels/prefill/pf_moe.metal:88-104);
+// padding positions are written as zeros. One warp per (row group, chunk).
 __global__ void __launch_bounds__(256) pf_prep_kernel(const PfParams p, const int *order) {
-  __shared__ __align__(16) unsigned char tile[2][4][2048];  // [gate | up][chunk of the pass][core matrix 16][row 8][16 bytes]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pos = blockIdx.x * 8 + warp, H = p.H;  // pos_cap is a multiple of 8
+  const int lane = threadIdx.x & 31, H = p.H, nc = H / 128;
+  const int job = blockIdx.x * 8 + (threadIdx.x >> 5), group = job / nc, chunk = job - group * nc;
+  if (group * 8 >= p.pos_cap) return;
+  const int pos = group * 8 + (lane >> 2);  // pos_cap is a multiple of 8
   const int slot = pos < p.off[p.E + 1] ? order[pos] : -1;
   const bool shared = slot >= p.S;
   const int t = slot < 0 ? 0 : shared ? slot - p.S : slot / p.topk;
   const int e = (slot < 0 || shared) ? 0 : p.seid[pos] - p.e0;
-  const __half *sg = shared ? p.sgt.suh : p.gate.suh + (size_t)e * H, *su = shared ? p.sup.suh : p.up.suh + (size_t)e * H;
-  const float *xr = p.x + (size_t)t * H;
-  const int j = lane >> 1, hsel = lane & 1;
-  const uint32_t woff = (uint32_t)(j * 128 + ((warp ^ (j & 7)) * 16) + hsel * 8);  // this lane's 8 bytes of its row's share of a chunk
-  for (int c0 = 0; c0 < H / 128; c0 += 4) {
-    float4 xv[4];
-    uint2 gs[4], us[4];
-    if (slot >= 0) {
+  float x[32], v[32];
+  quad_zero(x);
+  if (slot >= 0) quad_load(x, p.x + (size_t)t * H + chunk * 128, lane);
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int o = (min(c0 + i, H / 128 - 1)) * 128 + 4 * lane;
-        xv[i] = *reinterpret_cast<const float4 *>(xr + o);
-        gs[i] = *reinterpret_cast<const uint2 *>(sg + o);
-        us[i] = *reinterpret_cast<const uint2 *>(su + o);
-      }
-    }
+  for (int op = 0; op < 2; op++) {
+    const __half *s = (op == 0 ? (shared ? p.sgt.suh : p.gate.suh + (size_t)e * H) : (shared ? p.sup.suh : p.up.suh + (size_t)e * H)) + chunk * 128;
+    quad_zero(v);
+    if (slot >= 0) {  // (a padding row stays zero whatever the scales are)
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      uint2 go = make_uint2(0u, 0u), uo = make_uint2(0u, 0u);
-      if (slot >= 0 && c0 + i < H / 128) {  // uniform over the warp
-        const float4 g4 = mul4(xv[i], gs[i]), u4 = mul4(xv[i], us[i]);
-        float g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
-        fwht128_contig(g, lane, PF_HS);
-        fwht128_contig(u, lane, PF_HS);
-        go = pack4(g);
-        uo = pack4(u);
-      }
-      *reinterpret_cast<uint2 *>(&tile[0][i][woff]) = go;
-      *reinterpret_cast<uint2 *>(&tile[1][i][woff]) = uo;
+      for (int j = 0; j < 32; j++) v[j] = x[j];
+      quad_scale_in(v, s, lane);
     }
-    __syncthreads();
-    // 8 blocks of 2 KB (operand, chunk) = 1024 pieces of 16 bytes, four per thread; consecutive threads, consecutive bytes
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int idx = threadIdx.x + 256 * k, blk = idx >> 7, jj = (idx >> 3) & 15, r = idx & 7, op = blk >> 2, ci = blk & 3;
-      if (c0 + ci < H / 128) {
-        const uint4 v = *reinterpret_cast<const uint4 *>(&tile[op][ci][jj * 128 + ((r ^ (jj & 7)) * 16)]);
-        __half *dst = (op ? p.xh_u : p.xh_g) + (((size_t)blockIdx.x * (H >> 3) + (c0 + ci) * 16 + jj) << 6) + (r << 3);
-        *reinterpret_cast<uint4 *>(dst) = v;
-      }
-    }
-    __syncthreads();
+    fwht128_quad(v, lane, PF_HS);
+    quad_store_blocked(v, op == 0 ? p.xh_g : p.xh_u, pos, chunk, lane, H);
   }
 }
 
-// down operand: SwiGLU of the finished gate / up, times suh_down, H128, fp16 (reference pf_moe.metal:107-125)
+// down operand: SwiGLU of the finished gate / up, times suh_down, H128, fp16 (reference pf_moe.metal:107-125). One warp per
+// (row group, chunk); the down operand's transform takes its input in the order of quad_load, so the SwiGLU's values, which
+// come out contiguous, change places within the four lanes through shared memory.
 __global__ void __launch_bounds__(256) pf_mid_kernel(const PfParams p) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pos = blockIdx.x * 8 + warp, I = p.I;
-  if (pos >= p.pos_cap) return;
+  __shared__ __align__(16) float xch[8][32 * 36];  // per warp: a lane's 32 values, 16 bytes of padding (conflict-free 16-byte access)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, I = p.I, nc = I / 128;
+  const int job = blockIdx.x * 8 + warp, group = job / nc, chunk = job - group * nc;
+  if (group * 8 >= p.pos_cap) return;
+  const int pos = group * 8 + (lane >> 2);
   const int e = pos < p.off[p.E + 1] ? p.seid[pos] : -1;
-  if (e < 0) {
-    for (int c = 0; c < I / 128; c++) *reinterpret_cast<uint2 *>(blocked_lane_ptr(p.xh_d, pos, c, lane, I)) = make_uint2(0u, 0u);
-    return;
+  const bool live = e >= 0, shared = e == p.E;
+  const int el = shared || !live ? 0 : e - p.e0;
+  const int o = chunk * 128;
+  float g[32], u[32];
+  quad_zero(g);
+  quad_zero(u);
+  if (live) {
+    const float *raw = p.raw_gu + (size_t)pos * 2 * I + o;
+    quad_load(g, raw, lane);
+    quad_load(u, raw + I, lane);
   }
-  const bool shared = e == p.E;
-  const int el = shared ? 0 : e - p.e0;
-  const __half *svg = shared ? p.sgt.svh : p.gate.svh + (size_t)el * I, *svu = shared ? p.sup.svh : p.up.svh + (size_t)el * I;
-  const __half *sud = shared ? p.sdn.suh : p.down.suh + (size_t)el * I;
-  const float *raw = p.raw_gu + (size_t)pos * 2 * I;
-  for (int c0 = 0; c0 < I / 128; c0 += 2) {
-    float4 gr[2], ur[2];
-    uint2 s_g[2], s_u[2], s_d[2];
+  fwht128_quad(g, lane, PF_HS);
+  fwht128_quad(u, lane, PF_HS);
+  if (live) {
+    quad_scale_out(g, (shared ? p.sgt.svh : p.gate.svh + (size_t)el * I) + o, lane);
+    quad_scale_out(u, (shared ? p.sup.svh : p.up.svh + (size_t)el * I) + o, lane);
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int o = (min(c0 + i, I / 128 - 1)) * 128 + 4 * lane;
-      gr[i] = *reinterpret_cast<const float4 *>(raw + o);
-      ur[i] = *reinterpret_cast<const float4 *>(raw + I + o);
-      s_g[i] = *reinterpret_cast<const uint2 *>(svg + o);
-      s_u[i] = *reinterpret_cast<const uint2 *>(svu + o);
-      s_d[i] = *reinterpret_cast<const uint2 *>(sud + o);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      if (c0 + i < I / 128) {
-        float gv[4] = {gr[i].x, gr[i].y, gr[i].z, gr[i].w}, uv[4] = {ur[i].x, ur[i].y, ur[i].z, ur[i].w}, hh[4];
-        fwht128_contig(gv, lane, PF_HS);
-        fwht128_contig(uv, lane, PF_HS);
-        const float4 g4 = mul4(make_float4(gv[0], gv[1], gv[2], gv[3]), s_g[i]), u4 = mul4(make_float4(uv[0], uv[1], uv[2], uv[3]), s_u[i]);
-        const float4 d4 = mul4(make_float4(1.0f, 1.0f, 1.0f, 1.0f), s_d[i]);
-        hh[0] = g4.x / (1.0f + expf(-g4.x)) * u4.x * d4.x;
-        hh[1] = g4.y / (1.0f + expf(-g4.y)) * u4.y * d4.y;
-        hh[2] = g4.z / (1.0f + expf(-g4.z)) * u4.z * d4.z;
-        hh[3] = g4.w / (1.0f + expf(-g4.w)) * u4.w * d4.w;
-        fwht128_contig(hh, lane, PF_HS);
-        *reinterpret_cast<uint2 *>(blocked_lane_ptr(p.xh_d, pos, c0 + i, lane, I)) = pack4(hh);
-      }
-    }
+    for (int j = 0; j < 32; j++) g[j] = g[j] / (1.0f + expf(-g[j])) * u[j];
+    quad_scale_out(g, (shared ? p.sdn.suh : p.down.suh + (size_t)el * I) + o, lane);
   }
+  float *mine = &xch[warp][lane * 36];
+#pragma unroll
+  for (int c = 0; c < 8; c++) *reinterpret_cast<float4 *>(mine + 4 * c) = make_float4(g[4 * c], g[4 * c + 1], g[4 * c + 2], g[4 * c + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; i++) {  // element 16 i + 4 l + j: held by the lane of the quad whose run starts at 32 (i / 2)
+    const int owner = (lane & ~3) | ((i >> 2) & 1) | (((i >> 1) & 1) << 1);
+    const float4 a = *reinterpret_cast<const float4 *>(&xch[warp][owner * 36 + 16 * (i & 1) + 4 * (lane & 3)]);
+    g[4 * i] = a.x; g[4 * i + 1] = a.y; g[4 * i + 2] = a.z; g[4 * i + 3] = a.w;
+  }
+  fwht128_quad(g, lane, PF_HS);
+  quad_store_blocked(g, p.xh_d, pos, chunk, lane, I);
 }
 
-// finish: one CTA per (token, 512-column quarter), one warp per slot + one for the shared expert: every warp finishes its
-// slot's 4 chunks (H128, svh, routing weight) into shared memory, then the CTA sums the slots in slot order
-// (reference pf_moe.metal:129-161)
-constexpr int PF_FQ = 512;
+// finish: one CTA per (token, 1024 columns), one warp per slot + one for the shared expert: every warp finishes its slot's
+// eight chunks (H128, svh, routing weight) into shared memory, then the CTA sums the slots in slot order
+// (reference pf_moe.metal:129-161). A lane's 32 contiguous values go to shared memory in 16-byte pieces XORed with the number
+// of their 128-byte line, so neither the writes nor the reads of the sum meet in a bank.
+constexpr int PF_FQ = 1024;
 __global__ void __launch_bounds__(32 * 17) pf_finish_kernel(const PfParams p) {
   extern __shared__ __align__(16) float vals_dyn[];  // [slots][PF_FQ]; the block has one warp per slot, at least 4 warps
-  float(*vals)[PF_FQ] = reinterpret_cast<float(*)[PF_FQ]>(vals_dyn);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q0 = blockIdx.x * PF_FQ, t = blockIdx.y, H = p.H, k = p.topk;
   const int nslots = k + (p.has_shared ? 1 : 0);
-  const int nch = min(PF_FQ, H - q0) / 128;
-  bool have = false;
+  const int ncol = min(PF_FQ, H - q0);
   if (warp < nslots) {
     const bool shared = warp == k;
     const int pos = shared ? (t >= p.sh_row0 && t < p.sh_row0 + p.sh_rows ? p.off[p.E] + t - p.sh_row0 : -1) : p.inv[t * k + warp];
-    have = pos >= 0;
-  }
-  if (have) {
-    const bool shared = warp == k;
-    const int pos = shared ? p.off[p.E] + t - p.sh_row0 : p.inv[t * k + warp];
-    const int e = shared ? 0 : (int)p.route[(size_t)t * 2 * k + warp] - p.e0;
-    const float w = shared ? 1.0f / (1.0f + expf(-p.logits[(size_t)t * (p.E + 1) + p.E])) : __uint_as_float(p.route[(size_t)t * 2 * k + k + warp]);
-    const __half *sv = (shared ? p.sdn.svh : p.down.svh + (size_t)e * H) + q0;
-    const float *raw = p.raw_d + (size_t)pos * H + q0;
-    float4 rv[4];
-    uint2 sc[4];
+    const int o = (lane >> 2) * 128;  // this quad's chunk
+    const bool on = pos >= 0 && o < ncol;
+    float v[32];
+    quad_zero(v);
+    if (on) quad_load(v, p.raw_d + (size_t)pos * H + q0 + o, lane);
+    fwht128_quad(v, lane, PF_HS);
+    const int first = o + quad_first(lane);
+    if (on) {
+      const int e = shared ? 0 : (int)p.route[(size_t)t * 2 * k + warp] - p.e0;
+      const float w = shared ? 1.0f / (1.0f + expf(-p.logits[(size_t)t * (p.E + 1) + p.E])) : __uint_as_float(p.route[(size_t)t * 2 * k + k + warp]);
+      quad_scale_out(v, (shared ? p.sdn.svh : p.down.svh + (size_t)e * H) + q0 + o, lane);
+      if (shared) {
+        float4 *dst = reinterpret_cast<float4 *>(p.sho + (size_t)t * H + q0 + first);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int o = min(i, nch - 1) * 128 + 4 * lane;
-      rv[i] = *reinterpret_cast<const float4 *>(raw + o);
-      sc[i] = *reinterpret_cast<const uint2 *>(sv + o);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if (i < nch) {
-        float v[4] = {rv[i].x, rv[i].y, rv[i].z, rv[i].w};
-        fwht128_contig(v, lane, PF_HS);
-        const float4 f = mul4(make_float4(v[0], v[1], v[2], v[3]), sc[i]);
-        if (shared) *reinterpret_cast<float4 *>(p.sho + (size_t)t * H + q0 + i * 128 + 4 * lane) = f;
-        *reinterpret_cast<float4 *>(&vals[warp][i * 128 + 4 * lane]) = make_float4(f.x * w, f.y * w, f.z * w, f.w * w);
+        for (int c = 0; c < 8; c++) dst[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
       }
-    }
-  } else if (warp < nslots) {  // a slot computed on another rank, or a row whose shared expert runs elsewhere
 #pragma unroll
-    for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(&vals[warp][i * 128 + 4 * lane]) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      for (int j = 0; j < 32; j++) v[j] *= w;
+    }  // else: a slot computed on another rank, or a row whose shared expert runs elsewhere: zeros
+    float *line = vals_dyn + warp * PF_FQ + first;
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      *reinterpret_cast<float4 *>(line + 4 * (c ^ ((first >> 5) & 7))) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
   }
   __syncthreads();
-  const int c = threadIdx.x * 4;  // 128 threads cover the quarter
-  if (c >= nch * 128) return;
-  float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int s = 0; s < nslots; s++) {
-    const float4 v = *reinterpret_cast<const float4 *>(&vals[s][c]);
-    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  for (int c = threadIdx.x * 4; c < ncol; c += blockDim.x * 4) {
+    const int at = (c & ~31) + 4 * (((c >> 2) & 7) ^ ((c >> 5) & 7));
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int s = 0; s < nslots; s++) {
+      const float4 v = *reinterpret_cast<const float4 *>(vals_dyn + s * PF_FQ + at);
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
+    *reinterpret_cast<float4 *>(p.y + (size_t)t * H + q0 + c) = acc;
   }
-  *reinterpret_cast<float4 *>(p.y + (size_t)t * H + q0 + c) = acc;
 }
 
 // =============================================================================================== one Linear, many rows
@@ -734,27 +759,17 @@ __global__ void __launch_bounds__(32 * 17) pf_finish_kernel(const PfParams p) {
 // decodes W' densely once per chunk and runs an fp16 GEMM): the same grouped GEMM with a single group that holds all
 // rows, i.e. every tile is decoded once per 128 rows straight into the tensor core's operand layout.
 __global__ void __launch_bounds__(256) pfl_prep_kernel(const float *__restrict__ x, const __half *__restrict__ suh, __half *xh, int n, int n8, int in) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * 8 + warp;
-  if (r >= n8) return;
-  for (int c0 = 0; c0 < in / 128; c0 += 4) {
-    float4 xv[4];
-    uint2 sc[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int o = min(c0 + i, in / 128 - 1) * 128 + 4 * lane;
-      xv[i] = r < n ? *reinterpret_cast<const float4 *>(x + (size_t)r * in + o) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      sc[i] = *reinterpret_cast<const uint2 *>(suh + o);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if (c0 + i < in / 128) {
-        const float4 m = mul4(xv[i], sc[i]);
-        float v[4] = {m.x, m.y, m.z, m.w};
-        fwht128_contig(v, lane, PF_HS);
-        *reinterpret_cast<uint2 *>(blocked_lane_ptr(xh, r, c0 + i, lane, in)) = pack4(v);
-      }
-    }
+  const int lane = threadIdx.x & 31, nc = in / 128, job = blockIdx.x * 8 + (threadIdx.x >> 5), group = job / nc, chunk = job - group * nc;
+  if (group * 8 >= n8) return;
+  const int r = group * 8 + (lane >> 2);
+  float v[32];
+  quad_zero(v);
+  if (r < n) {
+    quad_load(v, x + (size_t)r * in + chunk * 128, lane);
+    quad_scale_in(v, suh + chunk * 128, lane);
   }
+  fwht128_quad(v, lane, PF_HS);
+  quad_store_blocked(v, xh, r, chunk, lane, in);
 }
 
 __global__ void pfl_items_kernel(PfItem *items, int *nitems, int n, int ncb) {
@@ -766,15 +781,21 @@ __global__ void pfl_items_kernel(PfItem *items, int *nitems, int n, int ncb) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *nitems = total;
 }
 
+// one warp per (row, eight chunks)
 __global__ void __launch_bounds__(256) pfl_finish_kernel(const float *__restrict__ raw, const __half *__restrict__ svh, float *y, int n, int out) {
-  const int lane = threadIdx.x & 31, nc = out / 128, job = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (job >= n * nc) return;
-  const int r = job / nc, o = (job - r * nc) * 128 + 4 * lane;
-  const float4 rv = *reinterpret_cast<const float4 *>(raw + (size_t)r * out + o);
-  const uint2 sc = *reinterpret_cast<const uint2 *>(svh + o);
-  float v[4] = {rv.x, rv.y, rv.z, rv.w};
-  fwht128_contig(v, lane, PF_HS);
-  *reinterpret_cast<float4 *>(y + (size_t)r * out + o) = mul4(make_float4(v[0], v[1], v[2], v[3]), sc);
+  const int lane = threadIdx.x & 31, nc = out / 128;
+  const long job = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 8 + (lane >> 2);
+  const int r = (int)(job / nc), o = (int)(job - (long)r * nc) * 128;
+  const bool on = r < n;
+  float v[32];
+  quad_zero(v);
+  if (on) quad_load(v, raw + (size_t)r * out + o, lane);
+  fwht128_quad(v, lane, PF_HS);
+  if (!on) return;
+  quad_scale_out(v, svh + o, lane);
+  float4 *dst = reinterpret_cast<float4 *>(y + (size_t)r * out + o + quad_first(lane));
+#pragma unroll
+  for (int c = 0; c < 8; c++) dst[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
 }
 
 size_t pf_linear_scratch_bytes(int in, int out, int n) {
@@ -794,7 +815,7 @@ void launch_pf_linear(const void *trellis, const void *suh, const void *svh, int
   PfItem *items = (PfItem *)(base + n8 * in * 2 + n8 * out * 4);
   int *nitems = (int *)((char *)items + passes * (out / PF_NCOL) * sizeof(PfItem));
   nitems = (int *)(((uintptr_t)nitems + 15) & ~(uintptr_t)15);
-  pfl_prep_kernel<<<(int)(n8 / 8), 256, 0, st>>>(x, (const __half *)suh, xh, n, (int)n8, in);
+  pfl_prep_kernel<<<(int)((n8 / 8 * (in / 128) + 7) / 8), 256, 0, st>>>(x, (const __half *)suh, xh, n, (int)n8, in);
   pfl_items_kernel<<<8, 256, 0, st>>>(items, nitems, n, out / PF_NCOL);
   IJ_CUDA(cudaGetLastError());
   PgGemm g{};
@@ -804,7 +825,7 @@ void launch_pf_linear(const void *trellis, const void *suh, const void *svh, int
   g.out[0] = raw;
   g.ldo = out; g.in = in; g.IT = in / 16; g.OT = out / 16; g.Kx = K; g.Ks = K;
   launch_pf_gemm(g, status, st);
-  pfl_finish_kernel<<<(n * (out / 128) + 7) / 8, 256, 0, st>>>(raw, (const __half *)svh, y, n, out);
+  pfl_finish_kernel<<<(int)(((size_t)n * (out / 128) + 63) / 64), 256, 0, st>>>(raw, (const __half *)svh, y, n, out);
   IJ_CUDA(cudaGetLastError());
 }
 
@@ -834,7 +855,7 @@ void launch_pf_moe(const PfParams &p, int *status, cudaStream_t st) {
   pf_blockscan_kernel<<<(p.E + 7) / 8, 256, 0, st>>>(p, p.hist, nb);
   pf_scan_kernel<<<1, 1024, 0, st>>>(p);
   pf_place_kernel<<<nb + nbs, 32, 0, st>>>(p, p.order, p.hist, nb);
-  pf_prep_kernel<<<groups, 256, 0, st>>>(p, p.order);
+  pf_prep_kernel<<<(groups * (p.H / 128) + 7) / 8, 256, 0, st>>>(p, p.order);
   IJ_CUDA(cudaGetLastError());
   PgGemm g{};
   g.items = p.items_gu; g.nitems = p.nitems;
@@ -843,7 +864,7 @@ void launch_pf_moe(const PfParams &p, int *status, cudaStream_t st) {
   g.out[0] = p.raw_gu; g.out[1] = p.raw_gu + p.I;
   g.ldo = 2 * p.I; g.in = p.H; g.IT = p.H / 16; g.OT = p.I / 16; g.Kx = p.Kx; g.Ks = p.has_shared ? p.Ks : p.Kx;
   launch_pf_gemm(g, status, st);
-  pf_mid_kernel<<<groups, 256, 0, st>>>(p);
+  pf_mid_kernel<<<(groups * (p.I / 128) + 7) / 8, 256, 0, st>>>(p);
   IJ_CUDA(cudaGetLastError());
   PgGemm d{};
   d.items = p.items_d; d.nitems = p.nitems + 1;
@@ -853,6 +874,8 @@ void launch_pf_moe(const PfParams &p, int *status, cudaStream_t st) {
   d.ldo = p.H; d.in = p.I; d.IT = p.I / 16; d.OT = p.H / 16; d.Kx = p.Kx; d.Ks = g.Ks;
   launch_pf_gemm(d, status, st);
   const int fslots = p.topk + (p.has_shared ? 1 : 0);  // one warp per slot; caller-routed pairs bring a single slot per row
+  // up to 17 slots of 4 KB (per device: every launch)
+  IJ_CUDA(cudaFuncSetAttribute(pf_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 17 * PF_FQ * 4));
   pf_finish_kernel<<<dim3((p.H + PF_FQ - 1) / PF_FQ, p.n), 32 * std::max(fslots, 4), (size_t)fslots * PF_FQ * 4, st>>>(p);
   IJ_CUDA(cudaGetLastError());
 }
