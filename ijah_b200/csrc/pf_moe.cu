@@ -10,38 +10,44 @@
 namespace ijah {
 
 // =============================================================================================== grouped trellis GEMM
-// out[pos][col] = sum_k act[pos][k] * W'_e[k][col] for one work item = (expert, <= 128 sorted rows, 256 output columns).
+// out[pos][col] = sum_k act[pos][k] * W'_e[k][col] for one work item = (expert, <= 256 sorted rows, 256 output columns).
 //
-// The contraction runs on the 5th-generation tensor core as D^T = W'^T * act^T: M = 128 output columns per accumulator
-// (two accumulators per item), N = the item's rows (16..128), K = 16 per instruction, accumulators in TMEM
-// (2 buffers x 2 x 128 columns = all 512, so the epilogue of one item overlaps the MMAs of the next).
-// One CTA per SM, warp-specialised:
-//   warp 0        producer: bulk-copies compressed tiles (4 k-tiles x 16 column tiles per stage) and the activations
-//                 (blocked layout, 1 KB per 8-row group per stage) into shared memory
-//   warp 1        issues tcgen05.mma (one thread) when a stage's decoded weights and activations are both present
+// The contraction runs on the 5th-generation tensor core as D^T = W'^T * act^T: M = 128 output columns per accumulator (two per
+// 128 rows), N = the rows (16..128), K = 16 per instruction. The accumulators of 128 rows are one half of TMEM: an item of at
+// most 128 rows takes one half, so the epilogue of one item overlaps the MMAs of the next; an item of more rows takes both and
+// multiplies every decoded weight with both groups of rows. One CTA per SM, warp-specialised:
+//   warp 0        weights: two tiled TMA copies per stage (4 k-tiles x 2 x 8 column tiles) into the ring
+//   warp 1        issues tcgen05.mma (one thread) when a stage's decoded weights and a group's activations are present
 //   warps 2-5     epilogue: tcgen05.ld the accumulators, store the live rows
 //   warps 6-21    decoders: each owns one of the 16 column tiles, decodes its tile of every k-tile with the same
 //                 register decode as the decode-width kernels and writes fp16 into the MMA's shared-memory layout
-// so every expert tile is decoded once per 128 rows instead of once per 16/32-row window.
+//   warp 22       activations: one bulk copy per stage and group of 128 rows (the operands are stored stage by stage)
+// so every expert tile is decoded once per 256 rows instead of once per 16/32-row window. The two kinds of copies have warps of
+// their own because each must run as far ahead as its own buffers allow: with one warp for both, the weights' ring was never
+// more than one stage ahead of the MMAs and a stage took 2.1 us at 128 rows (20 copies of 1 to 2.5 KB each) and 1.1 at 8.
 constexpr int PG_KS = 4;                      // k-tiles per stage
-constexpr int PG_RING = 4;                    // compressed-tile stages
-constexpr int PG_AB = 3;                      // decoded-weight / activation stages
-constexpr int PG_THREADS = 32 * 22;
+constexpr int PG_RING_MAX = 8;                // compressed-tile stages (as many as fit)
+constexpr int PG_A = 3;                       // decoded-weight stages
+constexpr int PG_B = 4;                       // activation slots (128 rows of one stage)
+constexpr int PG_THREADS = 32 * 23;
 constexpr int PG_A_STAGE = PG_KS * 2 * 4096;  // [ks][ng][khalf][16 groups][128 B]
-constexpr int PG_B_STAGE = 16 * 1024;         // [row group][8 k-chunks][128 B]
+constexpr int PG_B_SLOT = 16 * 1024;          // [row group][8 k-chunks][128 B]
 
 struct PgGemm {
+  alignas(64) CUtensorMap w_routed[2], w_shared[2];  // trellises per projection: boxes of 8 column tiles x PG_KS k-tiles
   const PfItem *items;
   const int *nitems;
-  const char *w_routed[2], *w_shared[2];  // trellis bases per projection
   const __half *act[2];                   // blocked activations per projection
   float *out[2];                          // output base per projection; element (pos, col) at out + pos * ldo + col
   int ldo, in, IT, OT, Kx, Ks;
+  int groups;                             // 8-row groups of the blocked operands
+  int ring;                               // ring stages
 };
 
 struct PgSmem {
-  uint64_t ring_full[PG_RING], ring_empty[PG_RING];
-  uint64_t a_full[PG_AB], b_full[PG_AB], ab_empty[PG_AB];
+  uint64_t ring_full[PG_RING_MAX], ring_empty[PG_RING_MAX];
+  uint64_t a_full[PG_A], a_empty[PG_A];
+  uint64_t b_full[PG_B], b_empty[PG_B];
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
 };
@@ -54,18 +60,18 @@ struct PgCursor {
 // All stages of one item for one decoder warp (column tile dw): straight-line code for one K, so that the lane's constants of
 // the other four do not compete for registers (with the choice of K inside the stage loop they spilled).
 template <int K>
-__device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, uint32_t ring_stage_bytes, uint32_t abuf, PgCursor &cu, int nst,
-                                               int dw, int lane, int *status) {
+__device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, uint32_t ring_stage_bytes, uint32_t nring, uint32_t abuf, PgCursor &cu,
+                                               int nst, int dw, int lane, int *status) {
   const typename Codec<K>::Lane L = Codec<K>::lane(lane);
   const McgConst mc = McgConst::load();
   const PairSum ps = PairSum::make(lane);
-  constexpr int KSTEP = 16 * Codec<K>::TILE_BYTES;
-  const uint32_t tile0 = ring + dw * Codec<K>::TILE_BYTES + L.o0, d1 = L.o1 - L.o0, d2 = L.o2 - L.o0;
+  constexpr int KSTEP = 8 * Codec<K>::TILE_BYTES;  // a ring stage is two boxes [k-tile][8 column tiles]
+  const uint32_t tile0 = ring + (uint32_t)((dw >> 3) * PG_KS * KSTEP + (dw & 7) * Codec<K>::TILE_BYTES) + L.o0, d1 = L.o1 - L.o0, d2 = L.o2 - L.o0;
   // lane (q, c) = (lane & 3, lane >> 2) writes k (2q, 2q + 1) and (2q + 8, 2q + 9) of columns c and c + 8
   const uint32_t dst0 = abuf + (uint32_t)((dw >> 3) * 4096 + (dw & 7) * 256 + lane * 4);
   const uint32_t bars = smem_u32(sm);
   const uint32_t rfull = bars + (uint32_t)offsetof(PgSmem, ring_full), rempty = bars + (uint32_t)offsetof(PgSmem, ring_empty);
-  const uint32_t afull = bars + (uint32_t)offsetof(PgSmem, a_full), aempty = bars + (uint32_t)offsetof(PgSmem, ab_empty);
+  const uint32_t afull = bars + (uint32_t)offsetof(PgSmem, a_full), aempty = bars + (uint32_t)offsetof(PgSmem, a_empty);
   const uint32_t lane0 = lane == 0 ? 1u : 0u;
 #pragma unroll 1
   for (int st = 0; st < nst; st++) {
@@ -94,8 +100,8 @@ __device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, 
     __syncwarp();
     mbar_arrive_if(afull + cu.as * 8u, lane0);
     mbar_arrive_if(rempty + cu.rs * 8u, lane0);
-    if (++cu.rs == PG_RING) { cu.rs = 0; cu.rph ^= 1u; }
-    if (++cu.as == PG_AB) { cu.as = 0; cu.aph ^= 1u; }
+    if (++cu.rs == nring) { cu.rs = 0; cu.rph ^= 1u; }
+    if (++cu.as == PG_A) { cu.as = 0; cu.aph ^= 1u; }
   }
   return true;
 }
@@ -104,16 +110,16 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
   extern __shared__ __align__(1024) unsigned char pf_smem[];
   unsigned char *smem = pf_smem;
   PgSmem *sm = reinterpret_cast<PgSmem *>(smem);
-  const int kmax = max(g.Kx, g.Ks);
-  const int ring_stage_bytes = PG_KS * 16 * 32 * kmax;
-  unsigned char *ring = smem + 1024;
-  unsigned char *abuf = ring + (size_t)PG_RING * ring_stage_bytes;  // ring_stage_bytes is a multiple of 2048
-  unsigned char *bbuf = abuf + (size_t)PG_AB * PG_A_STAGE;
+  const int ring_stage_bytes = PG_KS * 16 * 32 * max(g.Kx, g.Ks);
+  unsigned char *abuf = smem + 1024;
+  unsigned char *bbuf = abuf + (size_t)PG_A * PG_A_STAGE;
+  unsigned char *ring = bbuf + (size_t)PG_B * PG_B_SLOT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < PG_RING; s++) { mbar_init(&sm->ring_full[s], 1); mbar_init(&sm->ring_empty[s], 16); }
-    for (int s = 0; s < PG_AB; s++) { mbar_init(&sm->a_full[s], 16); mbar_init(&sm->b_full[s], 1); mbar_init(&sm->ab_empty[s], 1); }
+    for (int s = 0; s < g.ring; s++) { mbar_init(&sm->ring_full[s], 1); mbar_init(&sm->ring_empty[s], 16); }
+    for (int s = 0; s < PG_A; s++) { mbar_init(&sm->a_full[s], 16); mbar_init(&sm->a_empty[s], 1); }
+    for (int s = 0; s < PG_B; s++) { mbar_init(&sm->b_full[s], 1); mbar_init(&sm->b_empty[s], 1); }
     for (int b = 0; b < 2; b++) { mbar_init(&sm->acc_full[b], 1); mbar_init(&sm->acc_empty[b], 4); }
     mbar_fence_init();
   }
@@ -126,126 +132,150 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
   const int nst = g.IT / PG_KS;
 
   if (warp == 0) {
-    // ------------------------------------------------------------------------------------------ producer
-    int rs = 0, as = 0;
-    uint32_t rph = 0, aph = 0;
+    // ------------------------------------------------------------------------------------------ weights
+    int rs = 0;
+    uint32_t rph = 0;
+    const uint64_t pol = l2_evict_first_policy();
+    const uint32_t ring_a = smem_u32(ring);
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const PfItem im = g.items[it];
-      const int K = im.expert < 0 ? g.Ks : g.Kx;
-      const char *w = (im.expert < 0 ? g.w_shared[im.proj] : g.w_routed[im.proj] + (size_t)im.expert * g.IT * g.OT * 32 * K) +
-                      (size_t)im.ngpair * 16 * 32 * K;
-      const uint32_t kb = 16u * 32u * (uint32_t)K, kstride = (uint32_t)g.OT * 32u * (uint32_t)K;
-      const int ngroups = (im.nrows + 7) >> 3;
-      const __half *act = g.act[im.proj] + (size_t)(im.row0 >> 3) * (g.in >> 3) * 64;
+      const int expert = g.items[it].expert, proj = g.items[it].proj, ngpair = g.items[it].ngpair;
+      const int K = expert < 0 ? g.Ks : g.Kx, x0 = ngpair * 16 * 4 * K;
+      const CUtensorMap *map = expert < 0 ? &g.w_shared[proj] : &g.w_routed[proj];
+      const uint32_t box = (uint32_t)(PG_KS * 8 * 32) * (uint32_t)K;
       for (int st = 0; st < nst; st++) {
-        if (!mbar_wait(&sm->ring_empty[rs], rph ^ 1u, status, 11)) return;
-        if (lane == 0) mbar_arrive_expect_tx(&sm->ring_full[rs], PG_KS * kb);
+        if (!mbar_wait(&sm->ring_empty[rs], rph ^ 1u, status, 11)) goto out;
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(&sm->ring_full[rs]), dst = ring_a + (uint32_t)(rs * ring_stage_bytes);
+          mbar_arrive_expect_tx_a(bar, 2u * box);
+          tma_load_3d(dst, map, x0, st * PG_KS, max(expert, 0), bar, pol);
+          tma_load_3d(dst + box, map, x0 + 8 * 4 * K, st * PG_KS, max(expert, 0), bar, pol);
+        }
         __syncwarp();
-        if (lane < PG_KS)
-          bulk_g2s(ring + (size_t)rs * ring_stage_bytes + lane * kb, w + (size_t)(st * PG_KS + lane) * kstride, kb, &sm->ring_full[rs]);
-        if (++rs == PG_RING) { rs = 0; rph ^= 1u; }
-        if (!mbar_wait(&sm->ab_empty[as], aph ^ 1u, status, 12)) return;
-        if (lane == 0) mbar_arrive_expect_tx(&sm->b_full[as], (uint32_t)ngroups * 1024u);
-        __syncwarp();
-        if (lane < ngroups)
-          bulk_g2s(bbuf + (size_t)as * PG_B_STAGE + lane * 1024, act + ((size_t)lane * (g.in >> 3) + st * 8) * 64, 1024, &sm->b_full[as]);
-        if (++as == PG_AB) { as = 0; aph ^= 1u; }
+        if (++rs == g.ring) { rs = 0; rph ^= 1u; }
       }
+    }
+  } else if (warp == 22) {
+    // ------------------------------------------------------------------------------------------ activations
+    int bs = 0;
+    uint32_t bph = 0;
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+      const int row0 = g.items[it].row0, nrows = g.items[it].nrows;
+      const __half *act = g.act[g.items[it].proj] + (size_t)(row0 >> 3) * 512;
+      for (int st = 0; st < nst; st++)
+        for (int r0 = 0; r0 < nrows; r0 += PF_NTOK) {
+          if (!mbar_wait(&sm->b_empty[bs], bph ^ 1u, status, 12)) goto out;
+          if (lane == 0) {
+            const uint32_t bytes = (uint32_t)((min(PF_NTOK, nrows - r0) + 7) >> 3) * 1024u;
+            mbar_arrive_expect_tx(&sm->b_full[bs], bytes);
+            bulk_g2s(bbuf + (size_t)bs * PG_B_SLOT, act + ((size_t)st * g.groups + (r0 >> 3)) * 512, bytes, &sm->b_full[bs]);
+          }
+          __syncwarp();
+          if (++bs == PG_B) { bs = 0; bph ^= 1u; }
+        }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------------ MMA issuer
-    int as = 0, buf = 0;
-    uint32_t aph = 0, cph[2] = {0, 0};
+    int as = 0, bs = 0, half = 0;
+    uint32_t aph = 0, bph = 0, cph[2] = {0, 0};
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const PfItem im = g.items[it];
-      const uint32_t idesc = umma_idesc_f16(128, (im.nrows + 15) & ~15);
-      if (!mbar_wait(&sm->acc_empty[buf], cph[buf] ^ 1u, status, 13)) break;
+      const int nrows = g.items[it].nrows, nsub = nrows > PF_NTOK ? 2 : 1;
+      for (int s = 0; s < nsub; s++) {
+        const int h = half ^ s;
+        if (!mbar_wait(&sm->acc_empty[h], (h ? cph[1] : cph[0]) ^ 1u, status, 13)) goto out;
+        if (h) cph[1] ^= 1u; else cph[0] ^= 1u;
+      }
       tc_fence_after_sync();
       for (int st = 0; st < nst; st++) {
-        if (!mbar_wait(&sm->a_full[as], aph, status, 14)) goto done;
-        if (!mbar_wait(&sm->b_full[as], aph, status, 15)) goto done;
-        tc_fence_after_sync();
-        if (lane == 0) {
-          const uint32_t a0 = smem_u32(abuf + (size_t)as * PG_A_STAGE), b0 = smem_u32(bbuf + (size_t)as * PG_B_STAGE);
+        if (!mbar_wait(&sm->a_full[as], aph, status, 14)) goto out;
+        for (int s = 0; s < nsub; s++) {
+          if (!mbar_wait(&sm->b_full[bs], bph, status, 15)) goto out;
+          tc_fence_after_sync();
+          if (lane == 0) {
+            const uint32_t idesc = umma_idesc_f16(128, (min(PF_NTOK, nrows - s * PF_NTOK) + 15) & ~15);
+            const uint32_t a0 = smem_u32(abuf + (size_t)as * PG_A_STAGE), b0 = smem_u32(bbuf + (size_t)bs * PG_B_SLOT);
+            const uint32_t d0 = tmem + (uint32_t)(half ^ s) * 256u;
 #pragma unroll
-          for (int ks = 0; ks < PG_KS; ks++) {
-            const uint64_t bd = umma_smem_desc(b0 + ks * 256, 128, 1024);
+            for (int ks = 0; ks < PG_KS; ks++) {
+              const uint64_t bd = umma_smem_desc(b0 + ks * 256, 128, 1024);
 #pragma unroll
-            for (int ng = 0; ng < 2; ng++)
-              umma_f16_ss(tmem + (uint32_t)(buf * 2 + ng) * 128u, umma_smem_desc(a0 + (ks * 2 + ng) * 4096, 2048, 128), bd, idesc,
-                          (st > 0 || ks > 0) ? 1u : 0u);
+              for (int ng = 0; ng < 2; ng++)
+                umma_f16_ss(d0 + (uint32_t)ng * 128u, umma_smem_desc(a0 + (ks * 2 + ng) * 4096, 2048, 128), bd, idesc, (st > 0 || ks > 0) ? 1u : 0u);
+            }
+            umma_commit(&sm->b_empty[bs]);  // a slot may be overwritten once these MMAs have read it
+            if (s == nsub - 1) umma_commit(&sm->a_empty[as]);
+            if (st == nst - 1) umma_commit(&sm->acc_full[half ^ s]);
           }
-          umma_commit(&sm->ab_empty[as]);  // the stage may be overwritten once these MMAs have read it
-          if (st == nst - 1) umma_commit(&sm->acc_full[buf]);
+          __syncwarp();
+          if (++bs == PG_B) { bs = 0; bph ^= 1u; }
         }
-        __syncwarp();
-        if (++as == PG_AB) { as = 0; aph ^= 1u; }
+        if (++as == PG_A) { as = 0; aph ^= 1u; }
       }
-      cph[buf] ^= 1u;
-      buf ^= 1;
+      half ^= nsub & 1;
     }
-  done:;
   } else if (warp < 6) {
     // ------------------------------------------------------------------------------------------ epilogue
     const int qd = warp & 3;  // TMEM lanes 32 qd .. 32 qd + 31 are this warp's
-    int buf = 0;
+    int half = 0;
     uint32_t cph[2] = {0, 0};
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const PfItem im = g.items[it];
-      if (!mbar_wait(&sm->acc_full[buf], cph[buf], status, 16)) break;
-      tc_fence_after_sync();
-      float *out = g.out[im.proj] + (size_t)im.row0 * g.ldo + im.ngpair * PF_NCOL + qd * 32 + lane;
+      const int proj = g.items[it].proj, ngpair = g.items[it].ngpair, row0 = g.items[it].row0, nall = g.items[it].nrows;
+      for (int r0 = 0; r0 < nall; r0 += PF_NTOK) {
+        if (!mbar_wait(&sm->acc_full[half], half ? cph[1] : cph[0], status, 16)) goto out;
+        if (half) cph[1] ^= 1u; else cph[0] ^= 1u;
+        tc_fence_after_sync();
+        const int nrows = min(PF_NTOK, nall - r0);
+        float *out = g.out[proj] + (size_t)(row0 + r0) * g.ldo + ngpair * PF_NCOL + qd * 32 + lane;
 #pragma unroll 1
-      for (int ng = 0; ng < 2; ng++)
+        for (int ng = 0; ng < 2; ng++)
 #pragma unroll 1
-        for (int c0 = 0; c0 < im.nrows; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(buf * 2 + ng) * 128u + (uint32_t)c0, r);
-          float *o = out + (size_t)c0 * g.ldo + ng * 128;
-          uint32_t ld = (uint32_t)g.ldo;
-          asm volatile("" : "+r"(ld));  // (32 precomputed row offsets would not fit the registers)
+          for (int c0 = 0; c0 < nrows; c0 += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(half * 2 + ng) * 128u + (uint32_t)c0, r);
+            float *o = out + (size_t)c0 * g.ldo + ng * 128;
+            uint32_t ld = (uint32_t)g.ldo;
+            asm volatile("" : "+r"(ld));  // (32 precomputed row offsets would not fit the registers)
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
-            if (c0 + j < im.nrows) *o = __uint_as_float(r[j]);
-            o += ld;
+            for (int j = 0; j < 32; j++) {
+              if (c0 + j < nrows) *o = __uint_as_float(r[j]);
+              o += ld;
+            }
           }
-        }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm->acc_empty[buf]);
-      cph[buf] ^= 1u;
-      buf ^= 1;
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm->acc_empty[half]);
+        half ^= 1;
+      }
     }
   } else {
     // ------------------------------------------------------------------------------------------ decoders
     const int dw = warp - 6;
     PgCursor cu{0u, 0u, 0u, 0u};
-    const uint32_t ring_a = smem_u32(ring), abuf_a = smem_u32(abuf);
+    const uint32_t ring_a = smem_u32(ring), abuf_a = smem_u32(abuf), rsb = (uint32_t)ring_stage_bytes, nr = (uint32_t)g.ring;
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
       const int K = g.items[it].expert < 0 ? g.Ks : g.Kx;
       bool ok;
       switch (K) {
-        case 4: ok = pg_decode_item<4>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
-        case 5: ok = pg_decode_item<5>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
-        case 6: ok = pg_decode_item<6>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
-        case 7: ok = pg_decode_item<7>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
-        default: ok = pg_decode_item<8>(sm, ring_a, (uint32_t)ring_stage_bytes, abuf_a, cu, nst, dw, lane, status); break;
+        case 4: ok = pg_decode_item<4>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
+        case 5: ok = pg_decode_item<5>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
+        case 6: ok = pg_decode_item<6>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
+        case 7: ok = pg_decode_item<7>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
+        default: ok = pg_decode_item<8>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
       }
       if (!ok) break;
     }
   }
+out:
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-static size_t pg_smem_bytes(int kmax) { return 1024 + (size_t)PG_RING * PG_KS * 16 * 32 * kmax + (size_t)PG_AB * (PG_A_STAGE + PG_B_STAGE); }
-
-static void launch_pf_gemm(const PgGemm &g, int *status, cudaStream_t st) {
+static void launch_pf_gemm(PgGemm &g, int *status, cudaStream_t st) {
   IJ_CHECK(g.IT % PG_KS == 0 && g.OT % 16 == 0 && g.in % 64 == 0, "prefill GEMM needs in %% 64 == 0 and out %% 256 == 0 (in %d, out %d)", g.in, g.OT * 16);
-  const size_t smem = pg_smem_bytes(std::max(g.Kx, g.Ks));
+  const size_t fixed = 1024 + (size_t)PG_A * PG_A_STAGE + (size_t)PG_B * PG_B_SLOT, stage = (size_t)PG_KS * 16 * 32 * std::max(g.Kx, g.Ks);
+  g.ring = (int)std::min<size_t>(PG_RING_MAX, (226 * 1024 - fixed) / stage);  // 6 at K5, 4 at K8
   IJ_CUDA(cudaFuncSetAttribute(pf_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));  // per device: every launch
-  pf_gemm_kernel<<<sm_count(), PG_THREADS, smem, st>>>(g, status);
+  pf_gemm_kernel<<<sm_count(), PG_THREADS, fixed + g.ring * stage, st>>>(g, status);
   IJ_CUDA(cudaGetLastError());
 }
 
@@ -261,6 +291,7 @@ static void launch_pf_gemm(const PgGemm &g, int *status, cudaStream_t st) {
 constexpr int LG_T = 128, LG_K = 32, LG_LD = LG_K + 8;              // halfs per staged row
 constexpr int LG_PLANE = LG_T * LG_LD, LG_BUF = 4 * LG_PLANE;       // x hi, mid, lo, W
 constexpr int LG_SMEM = 2 * LG_BUF * 2;                             // bytes
+constexpr int LG_SPLITS = 8;                                        // most k-splits
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -282,19 +313,20 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t &hi, uint32_t 
   lo = bf16_rn_bits(a2) | (bf16_rn_bits(b2) << 16);
 }
 
-__global__ void __launch_bounds__(256) pf_logits_kernel(const PfParams p) {
+__global__ void __launch_bounds__(256) pf_logits_kernel(const PfParams p, float *part, int nk) {
   extern __shared__ __align__(16) unsigned char lg_smem[];
   uint16_t *sm = reinterpret_cast<uint16_t *>(lg_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t0 = blockIdx.x * LG_T, c0 = blockIdx.y * LG_T, H = p.H;
+  const int k_first = blockIdx.z * nk * LG_K;  // this split's first input
   const int wm = warp >> 1, wn = warp & 1;  // warp tile: tokens 32 wm .. +31, experts 64 wn .. +63
   // loads. x: thread -> rows (tid >> 3) + 32 j, floats 4 (tid & 7) .. +3; W: rows (tid >> 2) + 64 j, 16-byte chunk tid & 3
   const int xr = tid >> 3, xc = (tid & 7) * 4, wr = tid >> 2, wc = (tid & 3) * 8;
   const float *xsrc[4];
   const uint16_t *wsrc[2];
 #pragma unroll
-  for (int j = 0; j < 4; j++) xsrc[j] = p.x + (size_t)min(t0 + xr + 32 * j, p.n - 1) * H + xc;
+  for (int j = 0; j < 4; j++) xsrc[j] = p.x + (size_t)min(t0 + xr + 32 * j, p.n - 1) * H + k_first + xc;
 #pragma unroll
-  for (int j = 0; j < 2; j++) wsrc[j] = p.router + (size_t)min(c0 + wr + 64 * j, p.E - 1) * H + wc;
+  for (int j = 0; j < 2; j++) wsrc[j] = p.router + (size_t)min(c0 + wr + 64 * j, p.E - 1) * H + k_first + wc;
   float4 xv[4];
   auto load_x = [&](int ks) {
 #pragma unroll
@@ -335,7 +367,7 @@ __global__ void __launch_bounds__(256) pf_logits_kernel(const PfParams p) {
   // ldmatrix lane offsets (in halfs): A rows (lane & 15), k half (lane >> 4); B rows (lane & 7) + 8 ((lane >> 4) & 1), k half (lane >> 3) & 1
   const int a_off = (32 * wm + (lane & 15)) * LG_LD + (lane >> 4) * 8;
   const int b_off = (64 * wn + (lane & 7) + ((lane >> 4) & 1) * 8) * LG_LD + ((lane >> 3) & 1) * 8;
-  const int nk = H / LG_K;
+  nk = min(nk, (H - k_first) / LG_K);
   for (int ks = 0; ks < nk; ks++) {
     const int buf = ks & 1;
     if (ks + 1 < nk) {
@@ -378,7 +410,7 @@ __global__ void __launch_bounds__(256) pf_logits_kernel(const PfParams p) {
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         const int c = c0 + 64 * wn + 8 * j + 2 * q;
-        float *dst = p.logits + (size_t)t * (p.E + 1) + c;
+        float *dst = part + ((size_t)blockIdx.z * p.n + t) * (p.E + 1) + c;
         if (c < p.E) dst[0] = acc[i][j][2 * hh];
         if (c + 1 < p.E) dst[1] = acc[i][j][2 * hh + 1];
       }
@@ -386,13 +418,25 @@ __global__ void __launch_bounds__(256) pf_logits_kernel(const PfParams p) {
 }
 
 // top-k on the logits (ties -> lowest index), weights = softmax over the k selected; one warp per token
-__global__ void __launch_bounds__(256) pf_route_kernel(const PfParams p) {
+__global__ void __launch_bounds__(256) pf_route_kernel(const PfParams p, const float *part, int nsplit) {
   __shared__ float sl[8][1024];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x * 8 + warp;
   if (t >= p.n) return;
   float *s = sl[warp];
   const int E = p.E, k = p.topk;
-  for (int i = lane; i < E; i += 32) s[i] = p.logits[(size_t)t * (E + 1) + i];
+  if (nsplit == 1) {
+    for (int i = lane; i < E; i += 32) s[i] = p.logits[(size_t)t * (E + 1) + i];
+  } else {  // the router GEMM's k-splits, added in their order
+    for (int i = lane; i < E; i += 32) {
+      float v[LG_SPLITS];
+#pragma unroll
+      for (int j = 0; j < LG_SPLITS; j++) v[j] = j < nsplit ? part[((size_t)j * p.n + t) * (E + 1) + i] : 0.0f;
+#pragma unroll
+      for (int j = 1; j < LG_SPLITS; j++) v[0] += v[j];
+      s[i] = v[0];
+      p.logits[(size_t)t * (E + 1) + i] = v[0];
+    }
+  }
   if (p.has_shared) {  // the shared expert's gate logit: x[t] . w_sg
     float g = 0.0f;
     for (int i = lane * 8; i < p.H; i += 256) {
@@ -509,14 +553,14 @@ __global__ void __launch_bounds__(1024) pf_scan_kernel(const PfParams p) {
   __shared__ int wt[32], tot8, totp;
   __shared__ int s_pb[1024], s_off[1024], s_cnt[1024];
   const int e = threadIdx.x, E = p.E;
-  const int c = e < E ? p.cnt[e] : 0, c8 = (c + 7) & ~7, np = (c + PF_NTOK - 1) / PF_NTOK;
+  const int c = e < E ? p.cnt[e] : 0, c8 = (c + 7) & ~7, np = (c + PF_PASS - 1) / PF_PASS;
   const int o = block_excl_scan(c8, wt, &tot8);
   const int pb = block_excl_scan(np, wt, &totp);
   if (e < E) p.off[e] = o;
   s_pb[e] = e < E ? pb : 0x7FFFFFFF;
   s_off[e] = o;
   s_cnt[e] = c;
-  const int nsh = p.has_shared ? p.sh_rows : 0, shp = (nsh + PF_NTOK - 1) / PF_NTOK;
+  const int nsh = p.has_shared ? p.sh_rows : 0, shp = (nsh + PF_PASS - 1) / PF_PASS;
   if (e == 0) {
     p.off[E] = tot8;
     p.off[E + 1] = tot8 + ((nsh + 7) & ~7);
@@ -524,23 +568,28 @@ __global__ void __launch_bounds__(1024) pf_scan_kernel(const PfParams p) {
     p.nitems[1] = (totp + shp) * (p.H / PF_NCOL);
   }
   __syncthreads();
-  const int GU = p.I / PF_NCOL, DN = p.H / PF_NCOL;
-  auto emit = [&](int pass, int expert, int row0, int nrows) {
-    for (int j = 0; j < 2 * GU; j++) p.items_gu[pass * 2 * GU + j] = PfItem{expert, j / GU, j % GU, row0, nrows, {0, 0, 0}};
-    for (int j = 0; j < DN; j++) p.items_d[pass * DN + j] = PfItem{expert, 0, j, row0, nrows, {0, 0, 0}};
-  };
-  // one thread per pass: the expert of pass q is the last one whose first pass is <= q (experts without rows share the
-  // first-pass index of the next expert that has some)
-  for (int q = threadIdx.x; q < totp; q += blockDim.x) {
+  // one thread per item (a thread that writes all items of a pass one after the other made this kernel 35 to 53 us long).
+  // The expert of pass q is the last one whose first pass is <= q (experts without rows share the first-pass index of the
+  // next expert that has some); passes beyond the routed ones are the shared expert's.
+  auto pass_item = [&](int q, int proj, int ngpair) {
+    if (q >= totp) {
+      const int j = q - totp;
+      return PfItem{-1, proj, ngpair, tot8 + j * PF_PASS, min(PF_PASS, nsh - j * PF_PASS), {0, 0, 0}};
+    }
     int lo = 0, hi = 1024;  // first index with s_pb > q
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
       if (s_pb[mid] <= q) lo = mid + 1; else hi = mid;
     }
     const int ex = lo - 1, j = q - s_pb[ex];
-    emit(q, ex - p.e0, s_off[ex] + j * PF_NTOK, min(PF_NTOK, s_cnt[ex] - j * PF_NTOK));  // expert index into the local stacks
+    return PfItem{ex - p.e0, proj, ngpair, s_off[ex] + j * PF_PASS, min(PF_PASS, s_cnt[ex] - j * PF_PASS), {0, 0, 0}};  // expert index into the local stacks
+  };
+  const int GU = p.I / PF_NCOL, DN = p.H / PF_NCOL;
+  for (int i = threadIdx.x; i < (totp + shp) * 2 * GU; i += blockDim.x) {
+    const int q = i / (2 * GU), j = i - q * 2 * GU;
+    p.items_gu[i] = pass_item(q, j / GU, j % GU);
   }
-  for (int j = threadIdx.x; j < shp; j += blockDim.x) emit(totp + j, -1, tot8 + j * PF_NTOK, min(PF_NTOK, nsh - j * PF_NTOK));
+  for (int i = threadIdx.x; i < (totp + shp) * DN; i += blockDim.x) p.items_d[i] = pass_item(i / DN, 0, i % DN);
 }
 
 // order[pos] = slot (S + t for the shared expert's row of token t, -1 = padding), inv[slot] = pos, seid[pos] = expert
@@ -620,9 +669,9 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<const uint32_t *>(&h);
 }
-// fp16(v) into a blocked operand with `in` columns: chunk `chunk` of position pos
-__device__ __forceinline__ void quad_store_blocked(const float (&v)[32], __half *base, int pos, int chunk, int lane, int in) {
-  __half *dst = base + (((size_t)(pos >> 3) * (in >> 3) + chunk * 16 + (quad_first(lane) >> 3)) << 6) + ((pos & 7) << 3);
+// fp16(v) into a blocked operand of `groups` row groups: chunk `chunk` of position pos (a lane's run lies within one stage)
+__device__ __forceinline__ void quad_store_blocked(const float (&v)[32], __half *base, int pos, int chunk, int lane, int groups) {
+  __half *dst = base + blocked_index(pos, chunk * 128 + quad_first(lane), groups);
 #pragma unroll
   for (int c = 0; c < 4; c++)
     *reinterpret_cast<uint4 *>(dst + 64 * c) = make_uint4(pack2(v[8 * c], v[8 * c + 1]), pack2(v[8 * c + 2], v[8 * c + 3]),
@@ -657,7 +706,7 @@ __global__ void __launch_bounds__(256) pf_prep_kernel(const PfParams p, const in
       quad_scale_in(v, s, lane);
     }
     fwht128_quad(v, lane, PF_HS);
-    quad_store_blocked(v, op == 0 ? p.xh_g : p.xh_u, pos, chunk, lane, H);
+    quad_store_blocked(v, op == 0 ? p.xh_g : p.xh_u, pos, chunk, lane, p.pos_cap / 8);
   }
 }
 
@@ -702,7 +751,7 @@ __global__ void __launch_bounds__(256) pf_mid_kernel(const PfParams p) {
     g[4 * i] = a.x; g[4 * i + 1] = a.y; g[4 * i + 2] = a.z; g[4 * i + 3] = a.w;
   }
   fwht128_quad(g, lane, PF_HS);
-  quad_store_blocked(g, p.xh_d, pos, chunk, lane, I);
+  quad_store_blocked(g, p.xh_d, pos, chunk, lane, p.pos_cap / 8);
 }
 
 // finish: one CTA per (token, 1024 columns), one warp per slot + one for the shared expert: every warp finishes its slot's
@@ -769,14 +818,14 @@ __global__ void __launch_bounds__(256) pfl_prep_kernel(const float *__restrict__
     quad_scale_in(v, suh + chunk * 128, lane);
   }
   fwht128_quad(v, lane, PF_HS);
-  quad_store_blocked(v, xh, r, chunk, lane, in);
+  quad_store_blocked(v, xh, r, chunk, lane, n8 / 8);
 }
 
-__global__ void pfl_items_kernel(PfItem *items, int *nitems, int n, int ncb) {
-  const int passes = (n + PF_NTOK - 1) / PF_NTOK, total = passes * ncb;
+__global__ void pfl_items_kernel(PfItem *items, int *nitems, int n, int ncb, int rows) {
+  const int passes = (n + rows - 1) / rows, total = passes * ncb;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int pass = i / ncb, cb = i - pass * ncb;
-    items[i] = PfItem{-1, 0, cb, pass * PF_NTOK, min(PF_NTOK, n - pass * PF_NTOK), {0, 0, 0}};
+    items[i] = PfItem{-1, 0, cb, pass * rows, min(rows, n - pass * rows), {0, 0, 0}};
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *nitems = total;
 }
@@ -816,14 +865,19 @@ void launch_pf_linear(const void *trellis, const void *suh, const void *svh, int
   int *nitems = (int *)((char *)items + passes * (out / PF_NCOL) * sizeof(PfItem));
   nitems = (int *)(((uintptr_t)nitems + 15) & ~(uintptr_t)15);
   pfl_prep_kernel<<<(int)((n8 / 8 * (in / 128) + 7) / 8), 256, 0, st>>>(x, (const __half *)suh, xh, n, (int)n8, in);
-  pfl_items_kernel<<<8, 256, 0, st>>>(items, nitems, n, out / PF_NCOL);
+  // rows per item: 256 halve the decode, 128 make twice as many items; the fewer rounds of the persistent grid decide (an item of
+  // 256 rows is weighed as 1.25 of 128: the decode is the same, the MMAs and the results double)
+  const int ncb = out / PF_NCOL, sms = sm_count();
+  auto rounds = [&](int rows) { return ((n + rows - 1) / rows * ncb + sms - 1) / sms; };
+  const int rows = rounds(PF_PASS) * 1.25 <= rounds(PF_NTOK) ? PF_PASS : PF_NTOK;
+  pfl_items_kernel<<<8, 256, 0, st>>>(items, nitems, n, ncb, rows);
   IJ_CUDA(cudaGetLastError());
   PgGemm g{};
   g.items = items; g.nitems = nitems;
-  g.w_shared[0] = (const char *)trellis;
+  make_trellis_map(&g.w_shared[0], trellis, 1, in / 16, out / 16, K, PG_KS);
   g.act[0] = xh;
   g.out[0] = raw;
-  g.ldo = out; g.in = in; g.IT = in / 16; g.OT = out / 16; g.Kx = K; g.Ks = K;
+  g.groups = (int)(n8 / 8); g.ldo = out; g.in = in; g.IT = in / 16; g.OT = out / 16; g.Kx = K; g.Ks = K;
   launch_pf_gemm(g, status, st);
   pfl_finish_kernel<<<(int)(((size_t)n * (out / 128) + 63) / 64), 256, 0, st>>>(raw, (const __half *)svh, y, n, out);
   IJ_CUDA(cudaGetLastError());
@@ -843,8 +897,16 @@ void launch_pf_moe(const PfParams &p, int *status, cudaStream_t st) {
   IJ_CHECK(p.H % LG_K == 0, "prefill: hidden %d must be a multiple of %d", p.H, LG_K);
   if (!p.external_route) {
     IJ_CUDA(cudaFuncSetAttribute(pf_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LG_SMEM));
-    pf_logits_kernel<<<dim3((p.n + LG_T - 1) / LG_T, (p.E + LG_T - 1) / LG_T), 256, LG_SMEM, st>>>(p);
-    pf_route_kernel<<<(p.n + 7) / 8, 256, 0, st>>>(p);
+    // k-splits until every SM has two CTAs: a step of the k loop is a memory round trip, 64 of them in a row took 110 us for 333
+    // tokens (12 CTAs) and 117 for 4096 (128). The partial sums lie where the down products come later.
+    const int tiles = ((p.n + LG_T - 1) / LG_T) * ((p.E + LG_T - 1) / LG_T), steps = p.H / LG_K;
+    int nsplit = std::max(1, std::min(std::min(LG_SPLITS, 2 * sm_count() / tiles), steps));
+    while (nsplit > 1 && (size_t)nsplit * p.n * (p.E + 1) > (size_t)p.pos_cap * p.H) nsplit--;
+    const int nk = (steps + nsplit - 1) / nsplit;
+    nsplit = (steps + nk - 1) / nk;
+    float *part = nsplit > 1 ? p.raw_d : p.logits;
+    pf_logits_kernel<<<dim3((p.n + LG_T - 1) / LG_T, (p.E + LG_T - 1) / LG_T, nsplit), 256, LG_SMEM, st>>>(p, part, nk);
+    pf_route_kernel<<<(p.n + 7) / 8, 256, 0, st>>>(p, part, nsplit);
   } else {
     IJ_CHECK(!p.has_shared, "prefill: caller-routed pairs carry no shared expert");
   }
@@ -859,19 +921,29 @@ void launch_pf_moe(const PfParams &p, int *status, cudaStream_t st) {
   IJ_CUDA(cudaGetLastError());
   PgGemm g{};
   g.items = p.items_gu; g.nitems = p.nitems;
-  g.w_routed[0] = p.gate.trellis; g.w_routed[1] = p.up.trellis; g.w_shared[0] = p.sgt.trellis; g.w_shared[1] = p.sup.trellis;
+  const bool routed = p.ecount > 0;  // (no items name a stack that is not there)
+  const int HT = p.H / 16, IT = p.I / 16;
+  if (routed) {
+    make_trellis_map(&g.w_routed[0], p.gate.trellis, p.ecount, HT, IT, p.Kx, PG_KS);
+    make_trellis_map(&g.w_routed[1], p.up.trellis, p.ecount, HT, IT, p.Kx, PG_KS);
+  }
+  if (p.has_shared) {
+    make_trellis_map(&g.w_shared[0], p.sgt.trellis, 1, HT, IT, p.Ks, PG_KS);
+    make_trellis_map(&g.w_shared[1], p.sup.trellis, 1, HT, IT, p.Ks, PG_KS);
+  }
   g.act[0] = p.xh_g; g.act[1] = p.xh_u;
   g.out[0] = p.raw_gu; g.out[1] = p.raw_gu + p.I;
-  g.ldo = 2 * p.I; g.in = p.H; g.IT = p.H / 16; g.OT = p.I / 16; g.Kx = p.Kx; g.Ks = p.has_shared ? p.Ks : p.Kx;
+  g.groups = groups; g.ldo = 2 * p.I; g.in = p.H; g.IT = p.H / 16; g.OT = p.I / 16; g.Kx = p.Kx; g.Ks = p.has_shared ? p.Ks : p.Kx;
   launch_pf_gemm(g, status, st);
   pf_mid_kernel<<<(groups * (p.I / 128) + 7) / 8, 256, 0, st>>>(p);
   IJ_CUDA(cudaGetLastError());
   PgGemm d{};
   d.items = p.items_d; d.nitems = p.nitems + 1;
-  d.w_routed[0] = p.down.trellis; d.w_shared[0] = p.sdn.trellis;
+  if (routed) make_trellis_map(&d.w_routed[0], p.down.trellis, p.ecount, IT, HT, p.Kx, PG_KS);
+  if (p.has_shared) make_trellis_map(&d.w_shared[0], p.sdn.trellis, 1, IT, HT, p.Ks, PG_KS);
   d.act[0] = p.xh_d;
   d.out[0] = p.raw_d;
-  d.ldo = p.H; d.in = p.I; d.IT = p.I / 16; d.OT = p.H / 16; d.Kx = p.Kx; d.Ks = g.Ks;
+  d.groups = groups; d.ldo = p.H; d.in = p.I; d.IT = p.I / 16; d.OT = p.H / 16; d.Kx = p.Kx; d.Ks = g.Ks;
   launch_pf_gemm(d, status, st);
   const int fslots = p.topk + (p.has_shared ? 1 : 0);  // one warp per slot; caller-routed pairs bring a single slot per row
   // up to 17 slots of 4 KB (per device: every launch)

@@ -9,7 +9,8 @@
 
 namespace ijah {
 
-constexpr int PF_NTOK = 128;   // token rows per GEMM pass (the N of the MMA)
+constexpr int PF_NTOK = 128;   // token rows per accumulator (the N of the MMA)
+constexpr int PF_PASS = 256;   // token rows per work item: the weights of an item are decoded once for all of them
 constexpr int PF_NCOL = 256;   // output columns per work item (two M = 128 accumulators)
 
 // One pass of the grouped GEMM: rows [row0, row0 + nrows) of the sorted (8-row padded) position space, all of one
@@ -19,7 +20,7 @@ struct PfItem {
   int proj;     // gate/up launch: 0 gate, 1 up; down launch: 0
   int ngpair;   // which block of 256 output columns
   int row0;     // first position (multiple of 8)
-  int nrows;    // 1..PF_NTOK
+  int nrows;    // 1..PF_PASS
   int pad[3];
 };
 
@@ -44,9 +45,9 @@ struct PfParams {
   int *inv;              // [S] slot -> position
   int *order;            // [pos_cap] position -> slot (S + t = shared row of token t, -1 = padding), rewritten every run
   int *seid;             // [pos_cap] position -> expert (E = shared, -1 = padding), rewritten every run
-  __half *xh_g, *xh_u;   // [pos_cap / 8][H / 8][8][8] blocked operands (see blocked_index)
+  __half *xh_g, *xh_u;   // [H / 64][pos_cap / 8][8][8][8] blocked operands (see blocked_index)
   float *raw_gu;         // [pos_cap][2][I]
-  __half *xh_d;          // [pos_cap / 8][I / 8][8][8]
+  __half *xh_d;          // [I / 64][pos_cap / 8][8][8][8]
   float *raw_d;          // [pos_cap][H]
   PfItem *items_gu, *items_d;
   int *nitems;           // [2]: gate/up items, down items
@@ -54,10 +55,11 @@ struct PfParams {
   float *sho;            // [n][H] finished shared down (inspection)
 };
 
-// element (pos, k) of a blocked operand with `in` columns: core matrices of 8 positions x 8 k, 128 contiguous bytes each,
-// the in/8 core matrices of one 8-position group contiguous. A GEMM stage (8 k-chunks of one group) is 1 KB contiguous.
-__host__ __device__ inline size_t blocked_index(int pos, int k, int in) {
-  return (((size_t)(pos >> 3) * (in >> 3) + (k >> 3)) << 6) + ((pos & 7) << 3) + (k & 7);
+// element (pos, k) of a blocked operand of `groups` 8-position groups: core matrices of 8 positions x 8 k, 128 contiguous bytes
+// each; a GEMM stage (64 k = 8 core matrices) of one group is 1 KB contiguous, and the same stage of consecutive groups follows
+// on, so what a work item's rows take of a stage is one contiguous piece, one bulk copy.
+__host__ __device__ inline size_t blocked_index(int pos, int k, int groups) {
+  return ((size_t)(k >> 6) * groups + (pos >> 3)) * 512 + (((k >> 3) & 7) << 6) + ((pos & 7) << 3) + (k & 7);
 }
 
 size_t pf_pos_cap(int n, int topk, int E, bool has_shared);
