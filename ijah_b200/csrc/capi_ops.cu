@@ -56,7 +56,7 @@ Moe::Moe(const ne_moe_desc &d, int max_rows_) : desc(d), max_rows(max_rows_) {
   gush = (float *)al(R * 2 * I * 4);
   if (shared_q8) { q8_g = (float *)al(R * I * 4); q8_u = (float *)al(R * I * 4); q8_act = (float *)al(R * I * 4); }
   sho = (float *)al(R * H * 4);
-  counter = (unsigned *)al(16);
+  counter = (unsigned *)al((1 + MOE_ROW_GROUPS) * 4);
   x_stage = (float *)al(R * H * 4);
   y_stage = (float *)al(R * H * 4);
   status = device_status_word();

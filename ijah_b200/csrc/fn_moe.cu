@@ -13,7 +13,7 @@ namespace ijah {
 // the last CTA to arrive selects top-k on the logits, ties -> lowest index, w = exp(l - l_max) / sum over the k).
 constexpr int RT_WARPS = 8;    // expert rows per CTA (one per warp): every CTA stages all activation rows, so fewer, fuller CTAs read them less often
 constexpr int RT_THREADS = 256;
-constexpr int RT_RC = 8;       // activation rows per pass
+constexpr int RT_RC = 8;       // activation rows per CTA
 constexpr int RT_EMAX = 1024;  // experts the finisher covers (32 logits per lane)
 constexpr int RT_PMAX = 2048;  // (row, slot) pairs the finisher covers
 
@@ -285,16 +285,21 @@ __device__ __forceinline__ void router_dot(const uint4 (&wreg)[16], const float 
   }
 }
 
-// Dynamic shared memory: first the activation rows of one pass (RT_RC rows x H floats, shared by the CTA's expert
-// rows), later reused by the finisher (the plan's tables, then the pairs' expert ids).
+// One CTA per (eight experts, eight activation rows). The last CTA of a row group to arrive selects the top-k of its rows, one
+// warp each; the last row group to be selected builds the plan. Up to eight rows that is one CTA finishing everything; with one
+// CTA column that took all rows in passes of eight, the passes and the selection of 64 rows (eight after one another per warp)
+// cost 89 us.
+// Dynamic shared memory: first the activation rows (RT_RC rows x H floats, shared by the CTA's expert rows), later reused by
+// the finishers (the plan's tables, the pairs' expert ids, the candidate lists).
+// p.counter: [0] row groups selected, [1 + group] CTAs of the group that have arrived; all zero between launches.
 __global__ void __launch_bounds__(RT_THREADS) moe_router_kernel(const MoeParams p, int build_plan) {
   extern __shared__ __align__(16) float dyn[];
   __shared__ int s_last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * RT_WARPS + warp;
+  const int row = blockIdx.x * RT_WARPS + warp, r0 = blockIdx.y * RT_RC, nr = min(RT_RC, p.rows - r0);
   const int H = p.H, E = p.E;
-  const uint16_t *wr = warp >= RT_WARPS ? nullptr : row < E ? p.router + (size_t)row * H : (row == E ? p.sgate : nullptr);
-  // the expert's weight row stays in registers for all passes: H / 256 x 8 bf16 per lane (H <= 4096)
+  const uint16_t *wr = row < E ? p.router + (size_t)row * H : (row == E ? p.sgate : nullptr);
+  // the expert's weight row in registers: H / 256 x 8 bf16 per lane (H <= 4096)
   // (clamped addresses, no predicates: all 16 loads are in flight at once; the dot loop skips the chunks past H / 8)
   uint4 wreg[16];
   const uint4 *wsrc = reinterpret_cast<const uint4 *>(wr != nullptr ? wr : p.router);
@@ -302,24 +307,21 @@ __global__ void __launch_bounds__(RT_THREADS) moe_router_kernel(const MoeParams 
   for (int j = 0; j < 16; j++) wreg[j] = __ldg(wsrc + min(j * 32 + lane, H / 8 - 1));
   pdl_launch();
   pdl_wait();  // the router weights above are static; the activations may be the preceding kernel's output
-  for (int r0 = 0; r0 < p.rows; r0 += RT_RC) {
-    const int nr = min(RT_RC, p.rows - r0);
-    __syncthreads();
-    {  // asynchronous 16-byte copies: every thread's share is in flight at once
-      const uint32_t dst = smem_u32(dyn);
-      const float4 *src = reinterpret_cast<const float4 *>(p.x + (size_t)r0 * H);
-      // row t, floats [8c, 8c+4) go to float4 slot t * H/4 + c, floats [8c+4, 8c+8) to slot t * H/4 + H/8 + c: a warp's
-      // 16-byte reads of either half are then contiguous (no bank conflicts)
-      const int q = H / 4, h8 = H / 8;
-      for (int t = 0; t < nr; t++)
-        for (int w = threadIdx.x; w < q; w += blockDim.x) {
-          const int slot = t * q + (w & 1) * h8 + (w >> 1);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)slot * 16u), "l"(src + t * q + w) : "memory");
-        }
-      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    if (wr == nullptr) continue;
+  {  // asynchronous 16-byte copies: every thread's share is in flight at once
+    const uint32_t dst = smem_u32(dyn);
+    const float4 *src = reinterpret_cast<const float4 *>(p.x + (size_t)r0 * H);
+    // row t, floats [8c, 8c+4) go to float4 slot t * H/4 + c, floats [8c+4, 8c+8) to slot t * H/4 + H/8 + c: a warp's
+    // 16-byte reads of either half are then contiguous (no bank conflicts)
+    const int q = H / 4, h8 = H / 8;
+    for (int t = 0; t < nr; t++)
+      for (int w = threadIdx.x; w < q; w += blockDim.x) {
+        const int slot = t * q + (w & 1) * h8 + (w >> 1);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)slot * 16u), "l"(src + t * q + w) : "memory");
+      }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  }
+  __syncthreads();
+  if (wr != nullptr) {
     float acc[RT_RC];
     if (nr == 1) router_dot<1>(wreg, dyn, H, lane, nr, acc);
     else if (nr == 2) router_dot<2>(wreg, dyn, H, lane, nr, acc);
@@ -329,35 +331,50 @@ __global__ void __launch_bounds__(RT_THREADS) moe_router_kernel(const MoeParams 
     for (int t = 0; t < RT_RC; t++) {
       if (t < nr) {  // uniform
         const float v = warp_sum(acc[t]);
-        if (lane == 0 && row <= E) p.logits[(size_t)(r0 + t) * (E + 1) + row] = v;
+        if (lane == 0) p.logits[(size_t)(r0 + t) * (E + 1) + row] = v;
       }
     }
   }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(p.counter, 1u) == gridDim.x - 1 ? 1 : 0;
+  if (threadIdx.x == 0) s_last = atomicAdd(p.counter + 1 + blockIdx.y, 1u) == gridDim.x - 1 ? 1 : 0;
   __syncthreads();
   if (!s_last) return;  // the finisher reads the other CTAs' logits with L2 loads (ld.global.cg), past their fences
   unsigned char *tables = reinterpret_cast<unsigned char *>(dyn);
   int *sid = reinterpret_cast<int *>(tables + 16 * RT_EMAX);
   unsigned long long *lists = reinterpret_cast<unsigned long long *>(tables + 16 * RT_EMAX + 4 * RT_PMAX);
-  for (int r = warp; r < p.rows; r += RT_THREADS / 32) {
-    if (p.E <= 512) topk_row<16>(p, r, sid, lists + warp * 32, lane);
-    else topk_row<32>(p, r, sid, lists + warp * 32, lane);
+  static_assert(RT_RC == RT_THREADS / 32, "one warp per row of a group");
+  if (warp < nr) {
+    if (p.E <= 512) topk_row<16>(p, r0 + warp, sid, lists + warp * 32, lane);
+    else topk_row<32>(p, r0 + warp, sid, lists + warp * 32, lane);
+  }
+  if (threadIdx.x == 0) p.counter[1 + blockIdx.y] = 0u;
+  if (!build_plan) return;
+  if (gridDim.y > 1) {  // the plan takes the rows of all groups
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_last = atomicAdd(p.counter, 1u) == gridDim.y - 1 ? 1 : 0;
+      if (s_last) *p.counter = 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    const int k = p.topk;
+    for (int i = threadIdx.x; i < p.P; i += RT_THREADS) sid[i] = (int)__ldcg(p.route + (size_t)(i / k) * p.ldr + (i % k));
   }
   __syncthreads();
-  if (build_plan) build_plan_block(p, tables, sid);
-  if (threadIdx.x == 0) *p.counter = 0u;
+  build_plan_block(p, tables, sid);
 }
 
 void launch_moe_router(const MoeParams &p, bool build_plan, cudaStream_t st) {
   IJ_CHECK(p.E <= RT_EMAX && p.E % 32 == 0 && p.H % 256 == 0 && p.topk <= 32, "router: unsupported dims E %d H %d k %d", p.E, p.H, p.topk);
   IJ_CHECK(p.H <= 4096, "router: hidden %d > 4096", p.H);
   IJ_CHECK(p.P <= RT_PMAX, "router: %d (row, slot) pairs > %d", p.P, RT_PMAX);
-  const int grid = (p.E + 1 + RT_WARPS - 1) / RT_WARPS;
+  IJ_CHECK(p.rows <= RT_RC * MOE_ROW_GROUPS, "router: %d rows > %d", p.rows, RT_RC * MOE_ROW_GROUPS);
+  const dim3 grid((p.E + 1 + RT_WARPS - 1) / RT_WARPS, (p.rows + RT_RC - 1) / RT_RC);
   const size_t smem = std::max((size_t)std::min(p.rows, RT_RC) * p.H * 4, (size_t)16 * RT_EMAX + (size_t)RT_PMAX * 4 + 2048);  // tables, pair ids, candidate lists
   IJ_CUDA(cudaFuncSetAttribute(moe_router_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_RC * 4096 * 4));  // per device: every launch
-  launch_pdl(moe_router_kernel, dim3(grid), dim3(RT_THREADS), smem, st, p, build_plan ? 1 : 0);
+  launch_pdl(moe_router_kernel, grid, dim3(RT_THREADS), smem, st, p, build_plan ? 1 : 0);
 }
 
 // =============================================================================================== operand prep

@@ -14,6 +14,8 @@ struct Exl3Stack {
   const __half *svh;
 };
 
+constexpr int MOE_ROW_GROUPS = 8;  // groups of eight rows a launch can have (64 rows)
+
 struct MoeParams {
   int H, I, E, topk, Kx, Ks;
   int e0, ecount;     // local expert slice
@@ -42,7 +44,7 @@ struct MoeParams {
   float *gush;             // [rows][2 I]   finished shared gate | up
   float *sho;              // [rows][H]     finished shared down
   float *y;                // [rows][H]
-  unsigned *counter;
+  unsigned *counter;       // [1 + MOE_ROW_GROUPS], zero between launches
   // k-splits
   int S_gu, kc_gu, S_d, kc_d;
   // optional hyper-connection write (reference kernels/fn_moe.metal:446-450): h_out[r][s][c] = h[r][s][c] + y[r][c] * inj[r][s]
