@@ -12,25 +12,28 @@ namespace ijah {
 // =============================================================================================== grouped trellis GEMM
 // out[pos][col] = sum_k act[pos][k] * W'_e[k][col] for one work item = (expert, <= 256 sorted rows, 256 output columns).
 //
-// The contraction runs on the 5th-generation tensor core as D^T = W'^T * act^T: M = 128 output columns per accumulator (two per
-// 128 rows), N = the rows (16..128), K = 16 per instruction. The accumulators of 128 rows are one half of TMEM: an item of at
-// most 128 rows takes one half, so the epilogue of one item overlaps the MMAs of the next; an item of more rows takes both and
-// multiplies every decoded weight with both groups of rows. One CTA per SM, warp-specialised:
+// The contraction runs on the 5th-generation tensor core with the rows as M = 128 and all 256 columns as N, K = 16 per
+// instruction; the accumulator of 128 rows is one half of TMEM. An item of at most 128 rows takes one half, so the epilogue of
+// one item overlaps the MMAs of the next; an item of more rows takes both and multiplies every decoded weight with both groups
+// of rows. One CTA per SM, warp-specialised:
 //   warp 0        weights: two tiled TMA copies per stage (4 k-tiles x 2 x 8 column tiles) into the ring
-//   warp 1        issues tcgen05.mma (one thread) when a stage's decoded weights and a group's activations are present
+//   warp 1        issues tcgen05.mma (one thread) when a stage's decoded weights and activations are present
 //   warps 2-5     epilogue: tcgen05.ld the accumulators, store the live rows
 //   warps 6-21    decoders: each owns one of the 16 column tiles, decodes its tile of every k-tile with the same
 //                 register decode as the decode-width kernels and writes fp16 into the MMA's shared-memory layout
 //   warp 22       activations: one bulk copy per stage and group of 128 rows (the operands are stored stage by stage)
 // so every expert tile is decoded once per 256 rows instead of once per 16/32-row window. The two kinds of copies have warps of
-// their own because each must run as far ahead as its own buffers allow: with one warp for both, the weights' ring was never
-// more than one stage ahead of the MMAs and a stage took 2.1 us at 128 rows (20 copies of 1 to 2.5 KB each) and 1.1 at 8.
+// their own because each must run as far ahead as its own buffers allow.
+// Warp 1 shares its scheduler with decoders that are always ready, so each of its instructions costs several times its issue
+// slot: measured with cycle counters at 8 rows, eight MMAs of M = 128 columns x N rows with their descriptors took 634 cycles and the two
+// waits 150 each when there was nothing to wait for, together the 1110 cycles of a stage. Hence N = 256 (half the MMAs), descriptors that are
+// one addition away from the last, and all barriers of a stage polled at once by different lanes.
 constexpr int PG_KS = 4;                      // k-tiles per stage
 constexpr int PG_RING_MAX = 8;                // compressed-tile stages (as many as fit)
 constexpr int PG_A = 3;                       // decoded-weight stages
 constexpr int PG_B = 4;                       // activation slots (128 rows of one stage)
 constexpr int PG_THREADS = 32 * 23;
-constexpr int PG_A_STAGE = PG_KS * 2 * 4096;  // [ks][ng][khalf][16 groups][128 B]
+constexpr int PG_A_STAGE = PG_KS * 2 * 4096;  // [ks][khalf][32 groups of 8 columns][128 B]
 constexpr int PG_B_SLOT = 16 * 1024;          // [row group][8 k-chunks][128 B]
 
 struct PgGemm {
@@ -68,15 +71,17 @@ __device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, 
   constexpr int KSTEP = 8 * Codec<K>::TILE_BYTES;  // a ring stage is two boxes [k-tile][8 column tiles]
   const uint32_t tile0 = ring + (uint32_t)((dw >> 3) * PG_KS * KSTEP + (dw & 7) * Codec<K>::TILE_BYTES) + L.o0, d1 = L.o1 - L.o0, d2 = L.o2 - L.o0;
   // lane (q, c) = (lane & 3, lane >> 2) writes k (2q, 2q + 1) and (2q + 8, 2q + 9) of columns c and c + 8
-  const uint32_t dst0 = abuf + (uint32_t)((dw >> 3) * 4096 + (dw & 7) * 256 + lane * 4);
+  const uint32_t dst0 = abuf + (uint32_t)(dw * 256 + lane * 4);
   const uint32_t bars = smem_u32(sm);
   const uint32_t rfull = bars + (uint32_t)offsetof(PgSmem, ring_full), rempty = bars + (uint32_t)offsetof(PgSmem, ring_empty);
   const uint32_t afull = bars + (uint32_t)offsetof(PgSmem, a_full), aempty = bars + (uint32_t)offsetof(PgSmem, a_empty);
   const uint32_t lane0 = lane == 0 ? 1u : 0u;
+  const bool odd = lane & 1;
 #pragma unroll 1
   for (int st = 0; st < nst; st++) {
-    if (!mbar_wait_a(rfull + cu.rs * 8u, cu.rph, status, 17)) return false;
-    if (!mbar_wait_a(aempty + cu.as * 8u, cu.aph ^ 1u, status, 18)) return false;
+    // even lanes wait for the tiles, odd ones for the place to write to: one latency for both
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait_a(odd ? aempty + cu.as * 8u : rfull + cu.rs * 8u, odd ? cu.aph ^ 1u : cu.rph, status, 17))) return false;
+    __syncwarp();
     const uint32_t p0 = tile0 + cu.rs * ring_stage_bytes, p1 = p0 + d1, p2 = p0 + d2, dst = dst0 + cu.as * (uint32_t)PG_A_STAGE;
     static_assert(PG_KS == 4, "four k-tiles per stage");
     uint32_t w[4][3];
@@ -92,7 +97,7 @@ __device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, 
       round_pairs(hi, r[2], r[6], r[3], r[7], ps);
       const uint32_t d = dst + ks * 8192;  // (the offsets below are immediates)
       asm volatile(
-          "st.shared.u32 [%0], %1;\n\tst.shared.u32 [%0+2048], %2;\n\tst.shared.u32 [%0+128], %3;\n\tst.shared.u32 [%0+2176], %4;"
+          "st.shared.u32 [%0], %1;\n\tst.shared.u32 [%0+4096], %2;\n\tst.shared.u32 [%0+128], %3;\n\tst.shared.u32 [%0+4224], %4;"
           ::"r"(d), "r"(lo[0]), "r"(hi[0]), "r"(lo[1]), "r"(hi[1])
           : "memory");
     }
@@ -177,37 +182,49 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
     // ------------------------------------------------------------------------------------------ MMA issuer
     int as = 0, bs = 0, half = 0;
     uint32_t aph = 0, bph = 0, cph[2] = {0, 0};
+    const uint64_t w0 = umma_smem_desc(smem_u32(abuf), 4096, 128), x0 = umma_smem_desc(smem_u32(bbuf), 128, 1024);
+    const uint32_t afull = smem_u32(&sm->a_full[0]), bfull = smem_u32(&sm->b_full[0]);
+    constexpr uint32_t idesc = umma_idesc_f16(128, PF_NCOL);
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-      const int nrows = g.items[it].nrows, nsub = nrows > PF_NTOK ? 2 : 1;
+      const int nsub = g.items[it].nrows > PF_NTOK ? 2 : 1;
       for (int s = 0; s < nsub; s++) {
         const int h = half ^ s;
         if (!mbar_wait(&sm->acc_empty[h], (h ? cph[1] : cph[0]) ^ 1u, status, 13)) goto out;
         if (h) cph[1] ^= 1u; else cph[0] ^= 1u;
       }
-      tc_fence_after_sync();
       for (int st = 0; st < nst; st++) {
-        if (!mbar_wait(&sm->a_full[as], aph, status, 14)) goto out;
-        for (int s = 0; s < nsub; s++) {
-          if (!mbar_wait(&sm->b_full[bs], bph, status, 15)) goto out;
-          tc_fence_after_sync();
-          if (lane == 0) {
-            const uint32_t idesc = umma_idesc_f16(128, (min(PF_NTOK, nrows - s * PF_NTOK) + 15) & ~15);
-            const uint32_t a0 = smem_u32(abuf + (size_t)as * PG_A_STAGE), b0 = smem_u32(bbuf + (size_t)bs * PG_B_SLOT);
-            const uint32_t d0 = tmem + (uint32_t)(half ^ s) * 256u;
+        // lanes 0, 1, 2 (mod 4) poll the decoded weights and the activations of one or two groups of rows
+        const int bs1 = bs + 1 == PG_B ? 0 : bs + 1;
+        const uint32_t bph1 = bs + 1 == PG_B ? bph ^ 1u : bph;
+        const int which = lane & 3;
+        const uint32_t bar = which == 1 ? bfull + bs * 8u : which == 2 && nsub == 2 ? bfull + bs1 * 8u : afull + as * 8u;
+        const uint32_t par = which == 1 ? bph : which == 2 && nsub == 2 ? bph1 : aph;
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait_a(bar, par, status, 14))) goto out;
+        __syncwarp();
+        tc_fence_after_sync();
+        if (lane == 0) {
+          const uint64_t wd = w0 + (uint32_t)as * (uint32_t)(PG_A_STAGE >> 4);
+          uint64_t xd = x0 + (uint32_t)bs * (uint32_t)(PG_B_SLOT >> 4);
+          uint32_t d = tmem + (uint32_t)half * 256u;
+          umma_f16_ss(d, xd, wd, idesc, st > 0 ? 1u : 0u);
 #pragma unroll
-            for (int ks = 0; ks < PG_KS; ks++) {
-              const uint64_t bd = umma_smem_desc(b0 + ks * 256, 128, 1024);
+          for (int ks = 1; ks < PG_KS; ks++) umma_f16_ss(d, xd + ks * 16, wd + ks * 512, idesc, 1u);
+          umma_commit(&sm->b_empty[bs]);  // a slot may be overwritten once these MMAs have read it
+          if (nsub == 2) {
+            if (st == nst - 1) umma_commit(&sm->acc_full[half]);
+            xd = x0 + (uint32_t)bs1 * (uint32_t)(PG_B_SLOT >> 4);
+            d = tmem + (uint32_t)(half ^ 1) * 256u;
+            umma_f16_ss(d, xd, wd, idesc, st > 0 ? 1u : 0u);
 #pragma unroll
-              for (int ng = 0; ng < 2; ng++)
-                umma_f16_ss(d0 + (uint32_t)ng * 128u, umma_smem_desc(a0 + (ks * 2 + ng) * 4096, 2048, 128), bd, idesc, (st > 0 || ks > 0) ? 1u : 0u);
-            }
-            umma_commit(&sm->b_empty[bs]);  // a slot may be overwritten once these MMAs have read it
-            if (s == nsub - 1) umma_commit(&sm->a_empty[as]);
-            if (st == nst - 1) umma_commit(&sm->acc_full[half ^ s]);
+            for (int ks = 1; ks < PG_KS; ks++) umma_f16_ss(d, xd + ks * 16, wd + ks * 512, idesc, 1u);
+            umma_commit(&sm->b_empty[bs1]);
           }
-          __syncwarp();
-          if (++bs == PG_B) { bs = 0; bph ^= 1u; }
+          umma_commit(&sm->a_empty[as]);
+          if (st == nst - 1) umma_commit(&sm->acc_full[half ^ (nsub - 1)]);
         }
+        __syncwarp();
+        for (int s = 0; s < nsub; s++)
+          if (++bs == PG_B) { bs = 0; bph ^= 1u; }
         if (++as == PG_A) { as = 0; aph ^= 1u; }
       }
       half ^= nsub & 1;
@@ -223,23 +240,20 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
         if (!mbar_wait(&sm->acc_full[half], half ? cph[1] : cph[0], status, 16)) goto out;
         if (half) cph[1] ^= 1u; else cph[0] ^= 1u;
         tc_fence_after_sync();
-        const int nrows = min(PF_NTOK, nall - r0);
-        float *out = g.out[proj] + (size_t)(row0 + r0) * g.ldo + ngpair * PF_NCOL + qd * 32 + lane;
+        const int row = r0 + qd * 32 + lane;  // TMEM lane = row, column = column
+        if (r0 + qd * 32 < nall) {
+          float *o = g.out[proj] + (size_t)(row0 + row) * g.ldo + ngpair * PF_NCOL;
 #pragma unroll 1
-        for (int ng = 0; ng < 2; ng++)
-#pragma unroll 1
-          for (int c0 = 0; c0 < nrows; c0 += 32) {
+          for (int c0 = 0; c0 < PF_NCOL; c0 += 32) {
             uint32_t r[32];
-            tmem_ld_32x32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(half * 2 + ng) * 128u + (uint32_t)c0, r);
-            float *o = out + (size_t)c0 * g.ldo + ng * 128;
-            uint32_t ld = (uint32_t)g.ldo;
-            asm volatile("" : "+r"(ld));  // (32 precomputed row offsets would not fit the registers)
+            tmem_ld_32x32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)half * 256u + (uint32_t)c0, r);
+            if (row < nall) {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-              if (c0 + j < nrows) *o = __uint_as_float(r[j]);
-              o += ld;
+              for (int j = 0; j < 8; j++)
+                reinterpret_cast<uint4 *>(o + c0)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
             }
           }
+        }
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm->acc_empty[half]);
@@ -683,30 +697,40 @@ __device__ __forceinline__ void quad_zero(float (&v)[32]) {
 }
 
 // gate / up operands: xh[pos] = fp16(H128(x[token(pos)] * suh[expert(pos)])) (reference kernels/prefill/pf_moe.metal:88-104);
-// padding positions are written as zeros. One warp per (row group, chunk).
-__global__ void __launch_bounds__(256) pf_prep_kernel(const PfParams p, const int *order) {
-  const int lane = threadIdx.x & 31, H = p.H, nc = H / 128;
-  const int job = blockIdx.x * 8 + (threadIdx.x >> 5), group = job / nc, chunk = job - group * nc;
+// padding positions are written as zeros. One warp per (row group, PF_PREP_CHUNKS chunks): the rows' metadata is fetched once
+// and a chunk's activations are on their way while the chunk before is transformed.
+constexpr int PF_PREP_CHUNKS = 4;
+__global__ void __launch_bounds__(256, 2) pf_prep_kernel(const PfParams p, const int *order) {
+  const int lane = threadIdx.x & 31, H = p.H, nc = H / 128, runs = (nc + PF_PREP_CHUNKS - 1) / PF_PREP_CHUNKS;
+  const int job = blockIdx.x * 8 + (threadIdx.x >> 5), group = job / runs, c0 = (job - group * runs) * PF_PREP_CHUNKS;
   if (group * 8 >= p.pos_cap) return;
   const int pos = group * 8 + (lane >> 2);  // pos_cap is a multiple of 8
   const int slot = pos < p.off[p.E + 1] ? order[pos] : -1;
   const bool shared = slot >= p.S;
   const int t = slot < 0 ? 0 : shared ? slot - p.S : slot / p.topk;
   const int e = (slot < 0 || shared) ? 0 : p.seid[pos] - p.e0;
-  float x[32], v[32];
-  quad_zero(x);
-  if (slot >= 0) quad_load(x, p.x + (size_t)t * H + chunk * 128, lane);
+  const __half *const sg = shared ? p.sgt.suh : p.gate.suh + (size_t)e * H, *const su = shared ? p.sup.suh : p.up.suh + (size_t)e * H;
+  const float *const xr = p.x + (size_t)t * H;
+  const int c1 = min(nc, c0 + PF_PREP_CHUNKS);
+  float nx[32];
+  quad_zero(nx);
+  if (slot >= 0) quad_load(nx, xr + c0 * 128, lane);
+#pragma unroll 1
+  for (int c = c0; c < c1; c++) {
+    float x[32], v[32];
 #pragma unroll
-  for (int op = 0; op < 2; op++) {
-    const __half *s = (op == 0 ? (shared ? p.sgt.suh : p.gate.suh + (size_t)e * H) : (shared ? p.sup.suh : p.up.suh + (size_t)e * H)) + chunk * 128;
-    quad_zero(v);
-    if (slot >= 0) {  // (a padding row stays zero whatever the scales are)
+    for (int j = 0; j < 32; j++) x[j] = nx[j];
+    if (slot >= 0 && c + 1 < c1) quad_load(nx, xr + (c + 1) * 128, lane);
 #pragma unroll
-      for (int j = 0; j < 32; j++) v[j] = x[j];
-      quad_scale_in(v, s, lane);
-    }
+    for (int j = 0; j < 32; j++) v[j] = x[j];
+    if (slot >= 0) quad_scale_in(v, sg + c * 128, lane);  // (a padding row stays zero whatever the scales are)
     fwht128_quad(v, lane, PF_HS);
-    quad_store_blocked(v, op == 0 ? p.xh_g : p.xh_u, pos, chunk, lane, p.pos_cap / 8);
+    quad_store_blocked(v, p.xh_g, pos, c, lane, p.pos_cap / 8);
+#pragma unroll
+    for (int j = 0; j < 32; j++) v[j] = x[j];
+    if (slot >= 0) quad_scale_in(v, su + c * 128, lane);
+    fwht128_quad(v, lane, PF_HS);
+    quad_store_blocked(v, p.xh_u, pos, c, lane, p.pos_cap / 8);
   }
 }
 
@@ -917,7 +941,7 @@ void launch_pf_moe(const PfParams &p, int *status, cudaStream_t st) {
   pf_blockscan_kernel<<<(p.E + 7) / 8, 256, 0, st>>>(p, p.hist, nb);
   pf_scan_kernel<<<1, 1024, 0, st>>>(p);
   pf_place_kernel<<<nb + nbs, 32, 0, st>>>(p, p.order, p.hist, nb);
-  pf_prep_kernel<<<(groups * (p.H / 128) + 7) / 8, 256, 0, st>>>(p, p.order);
+  pf_prep_kernel<<<(groups * ((p.H / 128 + PF_PREP_CHUNKS - 1) / PF_PREP_CHUNKS) + 7) / 8, 256, 0, st>>>(p, p.order);
   IJ_CUDA(cudaGetLastError());
   PgGemm g{};
   g.items = p.items_gu; g.nitems = p.nitems;

@@ -21,7 +21,7 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t lbo_
 }
 
 // instruction descriptor: D = f32, A = B = f16, both K-major, M x N (M = 64 | 128, N multiple of 16 up to 256)
-__device__ __forceinline__ uint32_t umma_idesc_f16(int M, int N) {
+__host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N) {
   return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
