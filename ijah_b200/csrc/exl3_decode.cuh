@@ -243,6 +243,35 @@ __device__ __forceinline__ void fwht128_quad(float (&v)[32], int lane, float sca
   for (int p = 0; p < 32; p++) v[p] = o[p];
 }
 
+// The same for a chunk held as fwht128_quad leaves it (32 contiguous elements per lane), so that two transforms follow one another
+// without a change of places. Out: v[8 r + j] = element quad_run(lane, r) + j, four runs of eight.
+__device__ __forceinline__ int quad_run(int lane, int r) { return (r >> 1) * 64 + (r & 1) * 32 + (lane & 1) * 16 + ((lane >> 1) & 1) * 8; }
+__device__ __forceinline__ void fwht128_quad_runs(float (&v)[32], int lane, float scale) {
+#pragma unroll
+  for (int st = 1; st < 32; st <<= 1)
+#pragma unroll
+    for (int p = 0; p < 32; p++)
+      if ((p & st) == 0) {
+        const float a = v[p] + v[p + st], b = v[p] - v[p + st];
+        v[p] = a; v[p + st] = b;
+      }
+  const bool up1 = lane & 1, up2 = lane & 2;
+#pragma unroll
+  for (int p = 0; p < 16; p++) {  // bit 6, exchanged with bit 4
+    const float keep = up1 ? v[p + 16] : v[p], got = __shfl_xor_sync(0xFFFFFFFFu, up1 ? v[p] : v[p + 16], 1);
+    v[p] = keep + got; v[p + 16] = keep - got;
+  }
+#pragma unroll
+  for (int p = 0; p < 32; p++)
+    if ((p & 8) == 0) {  // bit 5, exchanged with bit 3
+      const float keep = up2 ? v[p + 8] : v[p], got = __shfl_xor_sync(0xFFFFFFFFu, up2 ? v[p] : v[p + 8], 2);
+      v[p] = keep + got; v[p + 8] = keep - got;
+    }
+  const float s1 = up1 ? -scale : scale, s2 = up2 ? -scale : scale, s12 = up1 != up2 ? -scale : scale;
+#pragma unroll
+  for (int p = 0; p < 32; p++) v[p] *= (p & 16) ? ((p & 8) ? s12 : s1) : ((p & 8) ? s2 : scale);
+}
+
 __host__ __device__ inline int had_size(int d) { return d % 128 == 0 ? 128 : d % 64 == 0 ? 64 : d % 32 == 0 ? 32 : 16; }
 
 }  // namespace ijah

@@ -19,20 +19,24 @@ namespace ijah {
 //   warp 0        weights: two tiled TMA copies per stage (4 k-tiles x 2 x 8 column tiles) into the ring
 //   warp 1        issues tcgen05.mma (one thread) when a stage's decoded weights and activations are present
 //   warps 2-5     epilogue: tcgen05.ld the accumulators, store the live rows
-//   warps 6-21    decoders: each owns one of the 16 column tiles, decodes its tile of every k-tile with the same
-//                 register decode as the decode-width kernels and writes fp16 into the MMA's shared-memory layout
-//   warp 22       activations: one bulk copy per stage and group of 128 rows (the operands are stored stage by stage)
+//   warps 6-29    decoders, three groups of eight: a group takes every third stage; each of its warps decodes two column tiles
+//                 of the stage's k-tiles with the same register decode as the decode-width kernels and writes fp16 into the
+//                 MMA's shared-memory layout
+//   warp 30       activations: one bulk copy per stage and group of 128 rows (the operands are stored stage by stage)
 // so every expert tile is decoded once per 256 rows instead of once per 16/32-row window. The two kinds of copies have warps of
 // their own because each must run as far ahead as its own buffers allow.
-// Warp 1 shares its scheduler with decoders that are always ready, so each of its instructions costs several times its issue
-// slot: measured with cycle counters at 8 rows, eight MMAs of M = 128 columns x N rows with their descriptors took 634 cycles and the two
-// waits 150 each when there was nothing to wait for, together the 1110 cycles of a stage. Hence N = 256 (half the MMAs), descriptors that are
-// one addition away from the last, and all barriers of a stage polled at once by different lanes.
+// What bounds it is the latency of one decoder's way through a stage, not a pipe: with sixteen decoders of four tiles per stage
+// (cycle counters, 8 rows) a stage took 2016 cycles, 1154 of them decoding, the rest waits, fence and arrivals, at 36 % of the
+// issue slots. Twenty-four decoders that pass the barriers once per eight tiles keep more work in flight. Warp 1 shares its
+// scheduler with them, so each of its instructions costs several times its issue slot (634 cycles for eight MMAs with M = 128
+// columns): hence N = 256, descriptors that are one addition away from the last and all barriers of a stage polled at once by
+// different lanes. The warps that mostly wait sleep between polls.
 constexpr int PG_KS = 4;                      // k-tiles per stage
 constexpr int PG_RING_MAX = 8;                // compressed-tile stages (as many as fit)
-constexpr int PG_A = 3;                       // decoded-weight stages
+constexpr int PG_A = 3;                       // decoded-weight stages = decoder groups
 constexpr int PG_B = 4;                       // activation slots (128 rows of one stage)
-constexpr int PG_THREADS = 32 * 23;
+constexpr int PG_DW = 8;                      // decoder warps per group; PG_A groups: group g fills decoded stage g
+constexpr int PG_THREADS = 32 * (7 + PG_A * PG_DW);
 constexpr int PG_A_STAGE = PG_KS * 2 * 4096;  // [ks][khalf][32 groups of 8 columns][128 B]
 constexpr int PG_B_SLOT = 16 * 1024;          // [row group][8 k-chunks][128 B]
 
@@ -55,58 +59,63 @@ struct PgSmem {
   uint32_t tmem_base;
 };
 
-// A decoder warp's view of the two rings
+// A decoder warp's view of the two rings: its group's next ring stage, the parities of that and of the group's decoded stage
 struct PgCursor {
-  uint32_t rs, as, rph, aph;
+  uint32_t rs, rph, aph;
 };
 
-// All stages of one item for one decoder warp (column tile dw): straight-line code for one K, so that the lane's constants of
-// the other four do not compete for registers (with the choice of K inside the stage loop they spilled).
+// The stages first, first + PG_A, .. of one item for one decoder warp (column tiles dw and dw + 8): straight-line code for one
+// K, so that the lane's constants of the other four do not compete for registers (with the choice of K inside the stage loop
+// they spilled).
 template <int K>
-__device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, uint32_t ring_stage_bytes, uint32_t nring, uint32_t abuf, PgCursor &cu,
-                                               int nst, int dw, int lane, int *status) {
+__device__ __forceinline__ bool pg_decode_item(const PgSmem *sm, uint32_t ring, uint32_t ring_stage_bytes, uint32_t nring, uint32_t abuf, int group,
+                                               PgCursor &cu, int first, int nst, int dw, int lane, int *status) {
   const typename Codec<K>::Lane L = Codec<K>::lane(lane);
   const McgConst mc = McgConst::load();
   const PairSum ps = PairSum::make(lane);
   constexpr int KSTEP = 8 * Codec<K>::TILE_BYTES;  // a ring stage is two boxes [k-tile][8 column tiles]
-  const uint32_t tile0 = ring + (uint32_t)((dw >> 3) * PG_KS * KSTEP + (dw & 7) * Codec<K>::TILE_BYTES) + L.o0, d1 = L.o1 - L.o0, d2 = L.o2 - L.o0;
+  const uint32_t tile0 = ring + (uint32_t)(dw * Codec<K>::TILE_BYTES) + L.o0, d1 = L.o1 - L.o0, d2 = L.o2 - L.o0;
   // lane (q, c) = (lane & 3, lane >> 2) writes k (2q, 2q + 1) and (2q + 8, 2q + 9) of columns c and c + 8
-  const uint32_t dst0 = abuf + (uint32_t)(dw * 256 + lane * 4);
+  const uint32_t dst = abuf + (uint32_t)(group * PG_A_STAGE + dw * 256 + lane * 4);
   const uint32_t bars = smem_u32(sm);
   const uint32_t rfull = bars + (uint32_t)offsetof(PgSmem, ring_full), rempty = bars + (uint32_t)offsetof(PgSmem, ring_empty);
-  const uint32_t afull = bars + (uint32_t)offsetof(PgSmem, a_full), aempty = bars + (uint32_t)offsetof(PgSmem, a_empty);
+  const uint32_t afull = bars + (uint32_t)offsetof(PgSmem, a_full) + group * 8u, aempty = bars + (uint32_t)offsetof(PgSmem, a_empty) + group * 8u;
   const uint32_t lane0 = lane == 0 ? 1u : 0u;
   const bool odd = lane & 1;
 #pragma unroll 1
-  for (int st = 0; st < nst; st++) {
+  for (int st = first; st < nst; st += PG_A) {
     // even lanes wait for the tiles, odd ones for the place to write to: one latency for both
-    if (!__all_sync(0xFFFFFFFFu, mbar_wait_a(odd ? aempty + cu.as * 8u : rfull + cu.rs * 8u, odd ? cu.aph ^ 1u : cu.rph, status, 17))) return false;
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait_a(odd ? aempty : rfull + cu.rs * 8u, odd ? cu.aph ^ 1u : cu.rph, status, 17))) return false;
     __syncwarp();
-    const uint32_t p0 = tile0 + cu.rs * ring_stage_bytes, p1 = p0 + d1, p2 = p0 + d2, dst = dst0 + cu.as * (uint32_t)PG_A_STAGE;
     static_assert(PG_KS == 4, "four k-tiles per stage");
-    uint32_t w[4][3];
-    w[0][0] = lds32<0 * KSTEP>(p0); w[0][1] = lds32<0 * KSTEP>(p1); w[0][2] = lds32<0 * KSTEP>(p2);
-    w[1][0] = lds32<1 * KSTEP>(p0); w[1][1] = lds32<1 * KSTEP>(p1); w[1][2] = lds32<1 * KSTEP>(p2);
-    w[2][0] = lds32<2 * KSTEP>(p0); w[2][1] = lds32<2 * KSTEP>(p1); w[2][2] = lds32<2 * KSTEP>(p2);
-    w[3][0] = lds32<3 * KSTEP>(p0); w[3][1] = lds32<3 * KSTEP>(p1); w[3][2] = lds32<3 * KSTEP>(p2);
 #pragma unroll
-    for (int ks = 0; ks < PG_KS; ks++) {
-      uint32_t r[8], lo[2], hi[2];
-      dec8_raw<K>(w[ks][0], w[ks][1], w[ks][2], L.a, mc, r);
-      round_pairs(lo, r[0], r[4], r[1], r[5], ps);
-      round_pairs(hi, r[2], r[6], r[3], r[7], ps);
-      const uint32_t d = dst + ks * 8192;  // (the offsets below are immediates)
-      asm volatile(
-          "st.shared.u32 [%0], %1;\n\tst.shared.u32 [%0+4096], %2;\n\tst.shared.u32 [%0+128], %3;\n\tst.shared.u32 [%0+4224], %4;"
-          ::"r"(d), "r"(lo[0]), "r"(hi[0]), "r"(lo[1]), "r"(hi[1])
-          : "memory");
+    for (int h = 0; h < 2; h++) {
+      const uint32_t p0 = tile0 + cu.rs * ring_stage_bytes + h * PG_KS * KSTEP, p1 = p0 + d1, p2 = p0 + d2;
+      uint32_t w[4][3];
+      w[0][0] = lds32<0 * KSTEP>(p0); w[0][1] = lds32<0 * KSTEP>(p1); w[0][2] = lds32<0 * KSTEP>(p2);
+      w[1][0] = lds32<1 * KSTEP>(p0); w[1][1] = lds32<1 * KSTEP>(p1); w[1][2] = lds32<1 * KSTEP>(p2);
+      w[2][0] = lds32<2 * KSTEP>(p0); w[2][1] = lds32<2 * KSTEP>(p1); w[2][2] = lds32<2 * KSTEP>(p2);
+      w[3][0] = lds32<3 * KSTEP>(p0); w[3][1] = lds32<3 * KSTEP>(p1); w[3][2] = lds32<3 * KSTEP>(p2);
+#pragma unroll
+      for (int ks = 0; ks < PG_KS; ks++) {
+        uint32_t r[8], lo[2], hi[2];
+        dec8_raw<K>(w[ks][0], w[ks][1], w[ks][2], L.a, mc, r);
+        round_pairs(lo, r[0], r[4], r[1], r[5], ps);
+        round_pairs(hi, r[2], r[6], r[3], r[7], ps);
+        const uint32_t d = dst + ks * 8192 + h * 2048;  // (the offsets below are immediates)
+        asm volatile(
+            "st.shared.u32 [%0], %1;\n\tst.shared.u32 [%0+4096], %2;\n\tst.shared.u32 [%0+128], %3;\n\tst.shared.u32 [%0+4224], %4;"
+            ::"r"(d), "r"(lo[0]), "r"(hi[0]), "r"(lo[1]), "r"(hi[1])
+            : "memory");
+      }
     }
     fence_proxy_async_smem();  // the tensor core reads what these ordinary stores wrote
     __syncwarp();
-    mbar_arrive_if(afull + cu.as * 8u, lane0);
+    mbar_arrive_if(afull, lane0);
     mbar_arrive_if(rempty + cu.rs * 8u, lane0);
-    if (++cu.rs == nring) { cu.rs = 0; cu.rph ^= 1u; }
-    if (++cu.as == PG_A) { cu.as = 0; cu.aph ^= 1u; }
+    cu.rs += PG_A;
+    if (cu.rs >= nring) { cu.rs -= nring; cu.rph ^= 1u; }
+    cu.aph ^= 1u;
   }
   return true;
 }
@@ -122,8 +131,8 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < g.ring; s++) { mbar_init(&sm->ring_full[s], 1); mbar_init(&sm->ring_empty[s], 16); }
-    for (int s = 0; s < PG_A; s++) { mbar_init(&sm->a_full[s], 16); mbar_init(&sm->a_empty[s], 1); }
+    for (int s = 0; s < g.ring; s++) { mbar_init(&sm->ring_full[s], 1); mbar_init(&sm->ring_empty[s], PG_DW); }
+    for (int s = 0; s < PG_A; s++) { mbar_init(&sm->a_full[s], PG_DW); mbar_init(&sm->a_empty[s], 1); }
     for (int s = 0; s < PG_B; s++) { mbar_init(&sm->b_full[s], 1); mbar_init(&sm->b_empty[s], 1); }
     for (int b = 0; b < 2; b++) { mbar_init(&sm->acc_full[b], 1); mbar_init(&sm->acc_empty[b], 4); }
     mbar_fence_init();
@@ -148,7 +157,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
       const CUtensorMap *map = expert < 0 ? &g.w_shared[proj] : &g.w_routed[proj];
       const uint32_t box = (uint32_t)(PG_KS * 8 * 32) * (uint32_t)K;
       for (int st = 0; st < nst; st++) {
-        if (!mbar_wait(&sm->ring_empty[rs], rph ^ 1u, status, 11)) goto out;
+        if (!mbar_wait_sleep(&sm->ring_empty[rs], rph ^ 1u, status, 11, 40)) goto out;
         if (lane == 0) {
           const uint32_t bar = smem_u32(&sm->ring_full[rs]), dst = ring_a + (uint32_t)(rs * ring_stage_bytes);
           mbar_arrive_expect_tx_a(bar, 2u * box);
@@ -159,7 +168,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
         if (++rs == g.ring) { rs = 0; rph ^= 1u; }
       }
     }
-  } else if (warp == 22) {
+  } else if (warp == 6 + PG_A * PG_DW) {
     // ------------------------------------------------------------------------------------------ activations
     int bs = 0;
     uint32_t bph = 0;
@@ -168,7 +177,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
       const __half *act = g.act[g.items[it].proj] + (size_t)(row0 >> 3) * 512;
       for (int st = 0; st < nst; st++)
         for (int r0 = 0; r0 < nrows; r0 += PF_NTOK) {
-          if (!mbar_wait(&sm->b_empty[bs], bph ^ 1u, status, 12)) goto out;
+          if (!mbar_wait_sleep(&sm->b_empty[bs], bph ^ 1u, status, 12, 40)) goto out;
           if (lane == 0) {
             const uint32_t bytes = (uint32_t)((min(PF_NTOK, nrows - r0) + 7) >> 3) * 1024u;
             mbar_arrive_expect_tx(&sm->b_full[bs], bytes);
@@ -202,7 +211,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
         if (!__all_sync(0xFFFFFFFFu, mbar_wait_a(bar, par, status, 14))) goto out;
         __syncwarp();
         tc_fence_after_sync();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint64_t wd = w0 + (uint32_t)as * (uint32_t)(PG_A_STAGE >> 4);
           uint64_t xd = x0 + (uint32_t)bs * (uint32_t)(PG_B_SLOT >> 4);
           uint32_t d = tmem + (uint32_t)half * 256u;
@@ -237,7 +246,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
       const int proj = g.items[it].proj, ngpair = g.items[it].ngpair, row0 = g.items[it].row0, nall = g.items[it].nrows;
       for (int r0 = 0; r0 < nall; r0 += PF_NTOK) {
-        if (!mbar_wait(&sm->acc_full[half], half ? cph[1] : cph[0], status, 16)) goto out;
+        if (!mbar_wait_sleep(&sm->acc_full[half], half ? cph[1] : cph[0], status, 16, 200)) goto out;
         if (half) cph[1] ^= 1u; else cph[0] ^= 1u;
         tc_fence_after_sync();
         const int row = r0 + qd * 32 + lane;  // TMEM lane = row, column = column
@@ -262,20 +271,23 @@ __global__ void __launch_bounds__(PG_THREADS, 1) pf_gemm_kernel(const __grid_con
     }
   } else {
     // ------------------------------------------------------------------------------------------ decoders
-    const int dw = warp - 6;
-    PgCursor cu{0u, 0u, 0u, 0u};
+    const int group = (warp - 6) / PG_DW, dw = (warp - 6) % PG_DW;
+    PgCursor cu{(uint32_t)group, 0u, 0u};
+    int first = group;  // the group's first stage of the item: the stages of all items are dealt to the groups in turn
     const uint32_t ring_a = smem_u32(ring), abuf_a = smem_u32(abuf), rsb = (uint32_t)ring_stage_bytes, nr = (uint32_t)g.ring;
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
       const int K = g.items[it].expert < 0 ? g.Ks : g.Kx;
       bool ok;
       switch (K) {
-        case 4: ok = pg_decode_item<4>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
-        case 5: ok = pg_decode_item<5>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
-        case 6: ok = pg_decode_item<6>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
-        case 7: ok = pg_decode_item<7>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
-        default: ok = pg_decode_item<8>(sm, ring_a, rsb, nr, abuf_a, cu, nst, dw, lane, status); break;
+        case 4: ok = pg_decode_item<4>(sm, ring_a, rsb, nr, abuf_a, group, cu, first, nst, dw, lane, status); break;
+        case 5: ok = pg_decode_item<5>(sm, ring_a, rsb, nr, abuf_a, group, cu, first, nst, dw, lane, status); break;
+        case 6: ok = pg_decode_item<6>(sm, ring_a, rsb, nr, abuf_a, group, cu, first, nst, dw, lane, status); break;
+        case 7: ok = pg_decode_item<7>(sm, ring_a, rsb, nr, abuf_a, group, cu, first, nst, dw, lane, status); break;
+        default: ok = pg_decode_item<8>(sm, ring_a, rsb, nr, abuf_a, group, cu, first, nst, dw, lane, status); break;
       }
       if (!ok) break;
+      first -= nst % PG_A;  // (stage nst + x of this item is stage x of the next)
+      if (first < 0) first += PG_A;
     }
   }
 out:
@@ -287,7 +299,7 @@ out:
 static void launch_pf_gemm(PgGemm &g, int *status, cudaStream_t st) {
   IJ_CHECK(g.IT % PG_KS == 0 && g.OT % 16 == 0 && g.in % 64 == 0, "prefill GEMM needs in %% 64 == 0 and out %% 256 == 0 (in %d, out %d)", g.in, g.OT * 16);
   const size_t fixed = 1024 + (size_t)PG_A * PG_A_STAGE + (size_t)PG_B * PG_B_SLOT, stage = (size_t)PG_KS * 16 * 32 * std::max(g.Kx, g.Ks);
-  g.ring = (int)std::min<size_t>(PG_RING_MAX, (226 * 1024 - fixed) / stage);  // 6 at K5, 4 at K8
+  g.ring = (int)std::min<size_t>(PG_RING_MAX, (226 * 1024 - fixed) / stage);  // 6 at K5, 4 at K8 (at least PG_A: a group's stages are PG_A apart)
   IJ_CUDA(cudaFuncSetAttribute(pf_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));  // per device: every launch
   pf_gemm_kernel<<<sm_count(), PG_THREADS, fixed + g.ring * stage, st>>>(g, status);
   IJ_CUDA(cudaGetLastError());
@@ -735,10 +747,8 @@ __global__ void __launch_bounds__(256, 2) pf_prep_kernel(const PfParams p, const
 }
 
 // down operand: SwiGLU of the finished gate / up, times suh_down, H128, fp16 (reference pf_moe.metal:107-125). One warp per
-// (row group, chunk); the down operand's transform takes its input in the order of quad_load, so the SwiGLU's values, which
-// come out contiguous, change places within the four lanes through shared memory.
-__global__ void __launch_bounds__(256) pf_mid_kernel(const PfParams p) {
-  __shared__ __align__(16) float xch[8][32 * 36];  // per warp: a lane's 32 values, 16 bytes of padding (conflict-free 16-byte access)
+// (row group, chunk).
+__global__ void __launch_bounds__(256, 3) pf_mid_kernel(const PfParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, I = p.I, nc = I / 128;
   const int job = blockIdx.x * 8 + warp, group = job / nc, chunk = job - group * nc;
   if (group * 8 >= p.pos_cap) return;
@@ -764,18 +774,11 @@ __global__ void __launch_bounds__(256) pf_mid_kernel(const PfParams p) {
     for (int j = 0; j < 32; j++) g[j] = g[j] / (1.0f + expf(-g[j])) * u[j];
     quad_scale_out(g, (shared ? p.sdn.suh : p.down.suh + (size_t)el * I) + o, lane);
   }
-  float *mine = &xch[warp][lane * 36];
+  fwht128_quad_runs(g, lane, PF_HS);
 #pragma unroll
-  for (int c = 0; c < 8; c++) *reinterpret_cast<float4 *>(mine + 4 * c) = make_float4(g[4 * c], g[4 * c + 1], g[4 * c + 2], g[4 * c + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 8; i++) {  // element 16 i + 4 l + j: held by the lane of the quad whose run starts at 32 (i / 2)
-    const int owner = (lane & ~3) | ((i >> 2) & 1) | (((i >> 1) & 1) << 1);
-    const float4 a = *reinterpret_cast<const float4 *>(&xch[warp][owner * 36 + 16 * (i & 1) + 4 * (lane & 3)]);
-    g[4 * i] = a.x; g[4 * i + 1] = a.y; g[4 * i + 2] = a.z; g[4 * i + 3] = a.w;
-  }
-  fwht128_quad(g, lane, PF_HS);
-  quad_store_blocked(g, p.xh_d, pos, chunk, lane, p.pos_cap / 8);
+  for (int r = 0; r < 4; r++)
+    *reinterpret_cast<uint4 *>(p.xh_d + blocked_index(pos, o + quad_run(lane, r), p.pos_cap / 8)) =
+        make_uint4(pack2(g[8 * r], g[8 * r + 1]), pack2(g[8 * r + 2], g[8 * r + 3]), pack2(g[8 * r + 4], g[8 * r + 5]), pack2(g[8 * r + 6], g[8 * r + 7]));
 }
 
 // finish: one CTA per (token, 1024 columns), one warp per slot + one for the shared expert: every warp finishes its slot's
@@ -783,7 +786,7 @@ __global__ void __launch_bounds__(256) pf_mid_kernel(const PfParams p) {
 // (reference pf_moe.metal:129-161). A lane's 32 contiguous values go to shared memory in 16-byte pieces XORed with the number
 // of their 128-byte line, so neither the writes nor the reads of the sum meet in a bank.
 constexpr int PF_FQ = 1024;
-__global__ void __launch_bounds__(32 * 17) pf_finish_kernel(const PfParams p) {
+__global__ void __launch_bounds__(32 * 17, 2) pf_finish_kernel(const PfParams p) {
   extern __shared__ __align__(16) float vals_dyn[];  // [slots][PF_FQ]; the block has one warp per slot, at least 4 warps
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q0 = blockIdx.x * PF_FQ, t = blockIdx.y, H = p.H, k = p.topk;
   const int nslots = k + (p.has_shared ? 1 : 0);

@@ -66,6 +66,15 @@ def test_rows_beyond_one_mma_tile(eng):
     check_block(eng, t, x, 6, max_rows=64)
 
 
+@pytest.mark.parametrize("rows", [7, 8, 9, 17, 64])
+def test_router_row_groups(eng, rows):
+    # groups of eight rows are selected by different CTAs, the last one builds the plan over all of them
+    rng = np.random.default_rng(900 + rows)
+    t = packgen.moe_layer(rng, hidden=512, inter=256, experts=64)
+    x = rng.standard_normal((rows, 512)).astype(np.float16).astype(np.float32)
+    check_block(eng, t, x, 5)
+
+
 def test_duplicate_rows_share_experts(eng):
     # identical rows route alike: every expert is used by all rows (the grouped path), outputs identical per row
     rng = np.random.default_rng(8)

@@ -95,6 +95,48 @@ def test_trunk_linear_prefill_matches_oracle_and_decode_path(eng, n_in, n_out, K
     assert np.array_equal(y, lin.prefill(xd).cpu().numpy()), "two runs must be bit-identical"
 
 
+@pytest.mark.parametrize("n_in,n_out,K,rows", [
+    (128, 256, 4, 65), (128, 256, 5, 128), (128, 512, 6, 129),  # two stages per item: one decoder group has none
+    (384, 256, 7, 256), (640, 256, 8, 257), (1024, 512, 5, 127),
+])
+def test_linear_prefill_at_the_edges_of_items_and_stages(eng, n_in, n_out, K, rows):
+    import torch
+    from ijah_b200 import engine as E
+    rng = np.random.default_rng(n_in + rows)
+    pk = packgen.exl3_linear(rng, n_in, n_out, K)
+    lin = E.Exl3Linear(eng, *pk)
+    x = rng.standard_normal((rows, n_in)).astype(np.float16).astype(np.float32)
+    y = lin.prefill(torch.from_numpy(x).cuda()).cpu().numpy()
+    want = np.concatenate([CO.linear_emul(*pk, x[i:i + 64]) for i in range(0, rows, 64)])
+    assert np.linalg.norm(y - want) / np.linalg.norm(want) < 5e-5  # the decode path's bound: f32 sums in another order
+    assert rel_max(y[-1], want[-1]) < 2e-4
+    assert eng.lib.ne_device_wait_status() == 0
+
+
+def test_prefill_items_of_two_row_groups(eng):
+    # 8 experts top-4 of 600 tokens: every expert has about 300 rows, so its items have two groups of 128 rows and a ragged rest;
+    # 150 tokens: one group; the router GEMM runs in eight k-splits. The decode path is the reference.
+    import torch
+    from ijah_b200 import engine as E
+    rng = np.random.default_rng(77)
+    t = packgen.moe_layer(rng, hidden=512, inter=256, experts=32)
+    pre = "language_model.model.layers.0.mlp."
+    from oracle import opref_port as O
+    w = O.bf16_bits_to_f32(t[pre + "gate.weight"][1]).copy()
+    x = rng.standard_normal((600, 512)).astype(np.float32)
+    x[:, 0] = 1.0
+    w[8:, 0] -= 8.0  # experts 8 .. 31 are never chosen
+    t[pre + "gate.weight"] = ("BF16", O.f32_to_bf16_bits(w))
+    x = x.astype(np.float16).astype(np.float32)
+    blk = E.MoeBlock(eng, t, top_k=4, max_rows=16)
+    xd = torch.from_numpy(x).cuda()
+    ref = np.concatenate([blk.forward(xd[i:i + 16]).cpu().numpy() for i in range(0, 600, 16)])
+    for n in (600, 150):
+        y = blk.prefill(xd[:n]).cpu().numpy()
+        assert rel_max(y, ref[:n]) < 2e-4
+    assert eng.lib.ne_device_wait_status() == 0
+
+
 def test_trunk_linear_prefill_rejects_unsupported_dims(eng):
     import torch
     from ijah_b200 import engine as E
