@@ -343,7 +343,6 @@ __global__ void __launch_bounds__(Q8S_THREADS, 1) q8_stream_kernel(const __grid_
       if (!mine) continue;  // another set's slab
       if (ok && !mbar_wait_a(smem_u32(&full[st]), ph, status, 2)) ok = false;
       if (!ok) continue;
-#ifndef Q8S_SKIP
       const uint32_t sbase = ring + st * (uint32_t)Q8S_STAGE_BYTES + a_rowoff;
       uint32_t a[4][4];
 #pragma unroll
@@ -386,9 +385,6 @@ __global__ void __launch_bounds__(Q8S_THREADS, 1) q8_stream_kernel(const __grid_
           tot[3] += sc1 * d[3] + bi1 * sbb;
         }
       }
-#else
-      if (lane == 0) mbar_arrive(&empty[st]);
-#endif
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&sempty[sb]);
