@@ -205,6 +205,14 @@ void Model::step(const int *tokens_host, int rows, int with_head, float *logits_
   IJ_CUDA(cudaEventRecord(ev0, stream));
   IJ_CUDA(cudaGraphLaunch(ex, stream));
   IJ_CUDA(cudaEventRecord(ev1, stream));
+  // the step is under way: touch the caller's logits pages meanwhile (a fresh buffer of 8 rows is 1187 page faults, which the copy would
+  // otherwise take one after the other when the step is done); their contents stay as they are
+  if (with_head && logits_host) {
+    volatile char *page = reinterpret_cast<volatile char *>(logits_host);
+    const size_t bytes = (size_t)rows * d.vocab * 4;
+    for (size_t i = 0; i < bytes; i += 4096) page[i] = page[i];
+    page[bytes - 1] = page[bytes - 1];
+  }
   if (with_head && next_host) IJ_CUDA(cudaMemcpyAsync(next_host, next, (size_t)rows * 4, cudaMemcpyDeviceToHost, stream));
   if (with_head && logits_host) IJ_CUDA(cudaMemcpyAsync(logits_host, logits, (size_t)rows * d.vocab * 4, cudaMemcpyDeviceToHost, stream));
   IJ_CUDA(cudaStreamSynchronize(stream));
