@@ -27,7 +27,8 @@ namespace ijah {
 // their own because each must run as far ahead as its own buffers allow.
 // What bounds it is the latency of one decoder's way through a stage, not a pipe: with sixteen decoders of four tiles per stage
 // (cycle counters, 8 rows) a stage took 2016 cycles, 1154 of them decoding, the rest waits, fence and arrivals, at 36 % of the
-// issue slots. Twenty-four decoders that pass the barriers once per eight tiles keep more work in flight. Warp 1 shares its
+// issue slots. Twenty-four decoders that pass the barriers once per eight tiles keep more work in flight (prefill block of
+// 333 tokens 1211 -> 1154 us); with the decode taken out of a copy the block took 874 us, with the MMAs 975: both sides are close. Warp 1 shares its
 // scheduler with them, so each of its instructions costs several times its issue slot (634 cycles for eight MMAs with M = 128
 // columns): hence N = 256, descriptors that are one addition away from the last and all barriers of a stage polled at once by
 // different lanes. The warps that mostly wait sleep between polls.
@@ -657,7 +658,8 @@ __global__ void __launch_bounds__(32) pf_place_kernel(const PfParams p, int *ord
 // The elementwise kernels below give four lanes one 128-element chunk of a row (fwht128_quad) and a warp the same chunk of the
 // eight rows of one row group of the blocked layout, whose rows all belong to one expert: what the warp writes of a core matrix
 // is then 128 contiguous bytes without a detour through shared memory, and the scale vectors are one broadcast per warp.
-// Prefill of 4096 tokens, Zipf routing: with one warp per row and 20 shuffles per chunk the three were bound by the shuffle pipe.
+// Prefill of 4096 tokens, Zipf routing: with one warp per row and 20 shuffles per chunk the three were bound by the shuffle pipe
+// and took 199 + 115 + 137 us; now 153 + 111 + 120, about twice what their f32 partial results and operands take at the DRAM rate.
 constexpr float PF_HS = 0.08838834764831845f;  // 1 / sqrt(128)
 
 // v[4 i + j] = element 16 i + 4 l + j of the lane's chunk of an f32 row
